@@ -8,7 +8,8 @@
 //     row (ConstructFundamentalSolutions + LUSolve, NonPeriodic2D_MPI.cpp:176-223,
 //     LU_Decomposition.cpp:78-108), the element-interface tridiagonal sweep with
 //     the Robin ends (NonPeriodic2D_MPI.cpp:265-295, 414-424) and the combination
-//     u = phi + zl ul + zr ur (:466-470), fused, one warp per complex row.
+//     u = phi + zl ul + zr ur (:466-470), fused, one warp per complex row (the LU
+//     method; fast-diagonalisation plans with several elements: helm_multi.cu).
 #include "helm_device.cuh"
 #include "helm_kernels.cuh"
 
@@ -1044,109 +1045,6 @@ __global__ void __launch_bounds__(ROW_WARPS * 32) rows_kernel(RowArgs a)
         const int r0 = a.grp_start[grp], r1 = a.grp_start[grp + 1];
         for (int rr = r0 + warp; rr < r1; rr += ROW_WARPS) {
             const long long rowoff = (long long)a.grp_rows[rr] * P;
-            if (ADJ && Ns > 1) {
-                // Transposed map of several elements.  Forward: per row the
-                // interface values z_0 .. z_Ns solve T z = h with h_0 = gl +
-                // al D0.phi_0, h_j = D0.phi_j - DN.phi_{j-1}, h_Ns = gr - ar
-                // DN.phi_{Ns-1}, and element j is u = phi_j + z_j ul + z_{j+1} ur
-                // (phi_j = A^-1 f_j).  Transposed: zbar_j gathers ubar at the
-                // nodes equal to z_j and ubar . ul / ur of the adjacent
-                // elements, w = T^-T zbar (the forward LU factors of T, used
-                // transposed), then phibar_j = ubar_j + (d0bar_j D0 + dNbar_j
-                // DN) on the interior, fbar_j = A^-T phibar_j, glbar = w_0,
-                // grbar = w_Ns (left in the boundary slots for the last pass).
-                const double* ul = a.fhom + (size_t)grp * 2 * P;
-                const double* ur = ul + P;
-                const double D0ul = a.fhoms[grp * 4 + 0], D0ur = a.fhoms[grp * 4 + 1];
-                const double DNul = a.fhoms[grp * 4 + 2], DNur = a.fhoms[grp * 4 + 3];
-                if (lane == 0)
-                    for (int j = 0; j <= Ns; ++j) { sNs[j * 6 + 0] = 0; sNs[j * 6 + 1] = 0; }
-                __syncwarp();
-                for (int jj = 0; jj < Ns; ++jj) {
-                    const CS* row = spec + (long long)jj * a.elem_stride + rowoff;
-                    TS slr = 0, sli = 0, srr = 0, sri = 0;
-#pragma unroll
-                    for (int s = 0; s < NSLOT; ++s) {
-                        const int i = lane + 32 * s;
-                        if (i < n) {
-                            const CS v = row[1 + i];
-                            const TS l = (TS)ul[1 + i], r = (TS)ur[1 + i];
-                            slr += l * v.x; sli += l * v.y;
-                            srr += r * v.x; sri += r * v.y;
-                        }
-                    }
-                    slr = warp_sum(slr); sli = warp_sum(sli);
-                    srr = warp_sum(srr); sri = warp_sum(sri);
-                    if (lane == 0) {
-                        const CS b0 = row[0], bN = row[P - 1];
-                        sNs[jj * 6 + 0] += b0.x + slr; sNs[jj * 6 + 1] += b0.y + sli;
-                        sNs[(jj + 1) * 6 + 0] += bN.x + srr; sNs[(jj + 1) * 6 + 1] += bN.y + sri;
-                    }
-                    __syncwarp();
-                }
-                if (lane == 0) {
-                    // T = L U without pivoting, as the forward sweep eliminates:
-                    // U diagonal b_j, super c_j; L sub q_j = T[j][j-1] / b_{j-1}.
-                    // U^T y = zbar (forward), then L^T w = y (backward).
-                    TS bp = 0, cp = 0, yr_ = 0, yi_ = 0;
-                    for (int j = 0; j <= Ns; ++j) {
-                        TS bj, cj;
-                        if (j == 0) {
-                            bj = (TS)(a.bl - a.al * D0ul);
-                            cj = (TS)(-a.al * D0ur);
-                        } else if (j < Ns) {
-                            bj = (TS)(DNur - D0ul) - ((TS)DNul / bp) * cp;
-                            cj = (TS)(-D0ur);
-                        } else {
-                            bj = (TS)(a.ar * DNur + a.br) - ((TS)(a.ar * DNul) / bp) * cp;
-                            cj = 0;
-                        }
-                        yr_ = (sNs[j * 6 + 0] - cp * yr_) / bj;
-                        yi_ = (sNs[j * 6 + 1] - cp * yi_) / bj;
-                        sNs[j * 6 + 2] = yr_; sNs[j * 6 + 3] = yi_; sNs[j * 6 + 4] = bj;
-                        bp = bj; cp = cj;
-                    }
-                    TS wr = sNs[Ns * 6 + 2], wi = sNs[Ns * 6 + 3];
-                    for (int j = Ns - 1; j >= 0; --j) {
-                        const TS q = (j + 1 < Ns ? (TS)DNul : (TS)(a.ar * DNul)) / sNs[j * 6 + 4];
-                        wr = sNs[j * 6 + 2] - q * wr;
-                        wi = sNs[j * 6 + 3] - q * wi;
-                        sNs[j * 6 + 2] = wr; sNs[j * 6 + 3] = wi;
-                    }
-                }
-                __syncwarp();
-                for (int jj = 0; jj < Ns; ++jj) {
-                    CS* row = spec + (long long)jj * a.elem_stride + rowoff;
-                    const TS w0r = sNs[jj * 6 + 2], w0i = sNs[jj * 6 + 3];
-                    const TS w1r = sNs[(jj + 1) * 6 + 2], w1i = sNs[(jj + 1) * 6 + 3];
-                    const TS s0 = jj == 0 ? (TS)a.al : (TS)1;           // d0bar = s0 w_jj
-                    const TS s1 = jj == Ns - 1 ? (TS)-a.ar : (TS)-1;    // dNbar = s1 w_{jj+1}
-                    TS fr[NSLOT], fi[NSLOT], xr[NSLOT], xi[NSLOT];
-#pragma unroll
-                    for (int s = 0; s < NSLOT; ++s) {
-                        const int i = lane + 32 * s;
-                        fr[s] = 0; fi[s] = 0;
-                        if (i < n) {
-                            const CS v = row[1 + i];
-                            const TS c0 = (TS)a.fd0[1 + i], cN = (TS)a.fdN[1 + i];
-                            fr[s] = v.x + s0 * w0r * c0 + s1 * w1r * cN;
-                            fi[s] = v.y + s0 * w0i * c0 + s1 * w1i * cN;
-                        }
-                    }
-                    solve_interior(fr, fi, xr, xi);
-#pragma unroll
-                    for (int s = 0; s < NSLOT; ++s) {
-                        const int i = lane + 32 * s;
-                        if (i < n) row[1 + i] = mk(xr[s], xi[s]);
-                    }
-                    if (lane == 0) {
-                        row[0] = jj == 0 ? mk(w0r, w0i) : mk((TS)0, (TS)0);
-                        row[P - 1] = jj == Ns - 1 ? mk(w1r, w1i) : mk((TS)0, (TS)0);
-                    }
-                }
-                __syncwarp();
-                continue;
-            }
             TS pr = 0, pi = 0;                        // running d/dy of the previous element (Ns > 1)
             TS rhs_r = 0, rhs_i = 0, bprev = 0, cprev = 0;
             TS d0r = 0, d0i = 0, dNr = 0, dNi = 0;
@@ -1442,8 +1340,8 @@ static int run_rows(const RowArgs& a, cudaStream_t s)
 template <int NSLOT>
 static int rows_dispatch_prec(int method, int prec, const RowArgs& a, cudaStream_t s)
 {
-    if (a.adjoint) {  // transposed solve: FDM only; several elements not periodic
-        if (method != 2 || (a.Ns > 1 && (a.periodic || !a.fhom))) return (int)cudaErrorInvalidValue;
+    if (a.adjoint) {  // transposed solve: FDM with one element (several: launch_multi)
+        if (method != 2 || a.Ns > 1) return (int)cudaErrorInvalidValue;
         if (prec == 0) return run_rows<double, double, NSLOT, 2, false, true>(a, s);
         if (prec == 1) return run_rows<float, float, NSLOT, 2, false, true>(a, s);
         return run_rows<double, float, NSLOT, 2, true, true>(a, s);

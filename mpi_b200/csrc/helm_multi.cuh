@@ -1,0 +1,53 @@
+// Row solves of plans with several GLL elements, fast-diagonalisation method
+// (helm_multi.cu).
+#pragma once
+#include <cuda_runtime.h>
+#include <vector>
+
+namespace helm {
+
+constexpr int MULTI_NMAX = 127;  // interior points per element the kernel covers
+
+// One solve of every spectrum row: Ns element vectors of n interior values, the
+// interface system that couples them, the combination.
+struct MultiArgs {
+    void* spec;               // complex [Ns][nrows][P] (elem_stride between elements)
+    long long elem_stride;    // complex elements
+    int P, n, Ns, nrows;
+    int rows_per_cta;         // set by launch_multi
+    const int* grp_of_row;    // shift group of each spectrum row
+    const double* m1;         // first transform, fragment order (multi_fragments)
+    const double* m2;         // second transform; forward: with the two end-slope rows
+    const double* lam;        // [n] eigenvalues of the interior operator
+    const double* sigma;      // [groups]
+    const double* hom;        // [groups][2][P] forward homogeneous solutions ul, ur
+    const double* homs;       // [groups][4] their end slopes D0.ul, D0.ur, DN.ul, DN.ur
+    // factors of the interface system (multi_interface): [groups][Ns + 1] reciprocal
+    // pivots; periodic: followed by the correction eta [Ns] and its weight
+    const double* itf;
+    const double* d0;         // [P] first and last row of D (adjoint)
+    const double* dN;
+    double al, ar;
+    int periodic, adjoint;
+};
+
+// Doubles of one transform with `outs` output rows in fragment order.
+inline size_t multi_fragment_doubles(int n, int outs)
+{
+    return (size_t)((n + 7) / 8) * 8 * ((outs + 7) / 8) * 8;
+}
+// Fragment order of the two transforms (m8n8k4 B operands): M1[j][k] (n x n)
+// read in natural k order, M2[i][j] (outs x n) in the k order in which the first
+// product leaves its results.
+std::vector<double> multi_fragments1(int n, const double* M1);
+std::vector<double> multi_fragments2(int n, int outs, const double* M2);
+
+// Reciprocal pivots of the interface system of one shift (and the periodic
+// correction) from the end slopes s[4]; out: Ns + 1 values, periodic 2 (Ns + 1).
+void multi_interface(int Ns, bool periodic, const double s[4], double al, double bl, double ar, double br,
+                     double* out);
+
+// spec_double: the spectrum holds doubles (else floats); arithmetic is FP64.
+int launch_multi(bool spec_double, MultiArgs a, cudaStream_t s);
+
+}  // namespace helm

@@ -12,6 +12,7 @@
 #include "../../include/helm_b200.h"
 #include "helm_fdm.cuh"
 #include "helm_kernels.cuh"
+#include "helm_multi.cuh"
 #include "helm_plan.hpp"
 #include "helm_eig.cuh"
 #include "helm_fd_refine.cuh"
@@ -239,31 +240,47 @@ static int setup_adjoint(Plan& p, const std::vector<double>& A0, const std::vect
     return HELM_OK;
 }
 
-// Transposed interior solves of a plan with several GLL elements (not
-// periodic): A^T = V^-T diag(lam) V^T and D2int^T for the refinement residual.
-// The interface system is transposed inside the row kernel from the forward
-// homogeneous solutions and end slopes, which such a plan already holds.
-static int setup_adjoint_multi(Plan& p, const std::vector<double>& A0, const std::vector<double>& V,
-                               const std::vector<double>& Vi, int prec_code)
+// Several GLL elements (helm_multi.cu): V^-1 and V (with the end-slope rows D0 V
+// and DN V below it) in fragment order, the factors of every shift's interface
+// system, and, for the adjoint of plans not periodic in the GLL direction, V^T
+// and V^-T (the interface system is transposed in the kernel).
+static int setup_multi(Plan& p, const std::vector<double>& V, const std::vector<double>& Vi,
+                       const std::vector<double>& homs)
 {
-    const int n = p.n, ld = p.ld;
-    std::vector<double> vtT((size_t)n * ld, 0.0), vinvtT((size_t)n * ld, 0.0), d2row((size_t)n * ld, 0.0);
-    for (int k = 0; k < n; ++k)
+    const int N = p.N, n = p.n, G = p.ngroups, M = p.Ns + 1, itf = p.periodic ? 2 * M : M;
+    const std::vector<double>& D = p.gll.D;
+    std::vector<double> vs((size_t)(n + 2) * n), vt((size_t)n * n), vit((size_t)n * n);
+    std::copy(V.begin(), V.end(), vs.begin());
+    for (int j = 0; j < n; ++j) {
+        long double s0 = 0, sN = 0;
         for (int i = 0; i < n; ++i) {
-            vtT[(size_t)k * ld + i] = V[k * n + i];
-            vinvtT[(size_t)k * ld + i] = Vi[k * n + i];
-            d2row[(size_t)k * ld + i] = A0[k * n + i];
+            s0 += (long double)D[i + 1] * V[(size_t)i * n + j];
+            sN += (long double)D[(size_t)(N - 1) * N + i + 1] * V[(size_t)i * n + j];
+            vt[(size_t)j * n + i] = V[(size_t)i * n + j];
+            vit[(size_t)j * n + i] = Vi[(size_t)i * n + j];
         }
-    auto up_mat = [&](const std::vector<double>& h, void** d) -> int {
-        if (prec_code == 0) return p.upload(d, h.data(), h.size() * sizeof(double));
-        std::vector<float> f(h.begin(), h.end());
-        return p.upload(d, f.data(), f.size() * sizeof(float));
-    };
+        vs[(size_t)n * n + j] = (double)s0;
+        vs[(size_t)(n + 1) * n + j] = (double)sN;
+    }
+    std::vector<double> f((size_t)G * itf);
+    for (int g = 0; g < G; ++g)
+        multi_interface(p.Ns, p.periodic, &homs[(size_t)g * 4], p.bc.alphal, p.bc.betal, p.bc.alphar, p.bc.betar,
+                        &f[(size_t)g * itf]);
+    std::vector<int> gor((size_t)p.nrows, 0);
+    for (int g = 0; g < G; ++g)
+        for (int rr = p.grp_start[g]; rr < p.grp_start[g + 1]; ++rr) gor[p.grp_rows[rr]] = g;
     int st;
-    if ((st = up_mat(vtT, &p.d_vtT))) return st;
-    if ((st = up_mat(vinvtT, &p.d_vinvtT))) return st;
-    if ((st = p.upload((void**)&p.d_d2row, d2row.data(), d2row.size() * sizeof(double)))) return st;
-    p.adj_ready = true;
+    auto up = [&](const std::vector<double>& h, double** d) { return p.upload((void**)d, h.data(), h.size() * sizeof(double)); };
+    if ((st = up(multi_fragments1(n, Vi.data()), &p.d_mm1))) return st;
+    if ((st = up(multi_fragments2(n, n + 2, vs.data()), &p.d_mm2))) return st;
+    if ((st = up(f, &p.d_itf))) return st;
+    if ((st = p.upload((void**)&p.d_grp_of_row, gor.data(), gor.size() * sizeof(int)))) return st;
+    if (!p.periodic) {
+        if ((st = up(multi_fragments1(n, vt.data()), &p.d_mm1_adj))) return st;
+        if ((st = up(multi_fragments2(n, n, vit.data()), &p.d_mm2_adj))) return st;
+        p.adj_ready = true;
+    }
+    p.multi = true;
     return HELM_OK;
 }
 
@@ -642,14 +659,16 @@ static int setup_plan(Plan& p)
         if ((st = up_mat(dinv, &p.d_dinv))) return st;
         if ((st = p.upload((void**)&p.d_perm, perm.data(), perm.size()))) return st;
     } else {
-        std::vector<double> vinvT((size_t)n * ld, 0.0), vT((size_t)n * ld, 0.0);
-        for (int k = 0; k < n; ++k)
-            for (int i = 0; i < n; ++i) {
-                vinvT[(size_t)k * ld + i] = Vi[i * n + k];
-                vT[(size_t)k * ld + i] = V[i * n + k];
-            }
-        if ((st = up_mat(vinvT, &p.d_vinvT))) return st;
-        if ((st = up_mat(vT, &p.d_vT))) return st;
+        if (p.Ns == 1) {
+            std::vector<double> vinvT((size_t)n * ld, 0.0), vT((size_t)n * ld, 0.0);
+            for (int k = 0; k < n; ++k)
+                for (int i = 0; i < n; ++i) {
+                    vinvT[(size_t)k * ld + i] = Vi[i * n + k];
+                    vT[(size_t)k * ld + i] = V[i * n + k];
+                }
+            if ((st = up_mat(vinvT, &p.d_vinvT))) return st;
+            if ((st = up_mat(vT, &p.d_vT))) return st;
+        }
         if ((st = p.upload((void**)&p.d_lam, lam.data(), lam.size() * sizeof(double)))) return st;
     }
     p.h_lam = lam;
@@ -658,8 +677,8 @@ static int setup_plan(Plan& p)
     if (!lu && p.Ns == 1) {
         if (p.packed_elems == 0 && (st = setup_adjoint(p, A0, lam, V, Vi, prec_code, homs))) return st;
         if ((st = setup_fast(p, A0, prec_code))) return st;
-    } else if (!lu && !p.periodic && p.packed_elems == 0 && p.batch == 1) {
-        if ((st = setup_adjoint_multi(p, A0, V, Vi, prec_code))) return st;
+    } else if (!lu) {
+        if ((st = setup_multi(p, V, Vi, homs))) return st;
     }
     if (!p.fast && rows_smem_bytes(p.method, prec_code, n, p.ld) > kMaxSmemPerBlock) {
         g_last_error = "GLL size too large for the row-solve kernel at this precision";
@@ -882,10 +901,6 @@ static int run_pipeline(Plan& p, const void* in, const double* gl, const double*
         r.d0 = p.d_c0;
         r.dN = p.d_cN;
         r.d2t = p.d_d2row;
-        r.fhom = p.d_hom;
-        r.fhoms = p.d_homs;
-        r.fd0 = p.d_d0;
-        r.fdN = p.d_dN;
     }
     r.periodic = p.periodic ? 1 : 0;
     const int prec = p.precision == HELM_FP64 ? 0 : (p.precision == HELM_FP32 ? 1 : 2);
@@ -950,6 +965,29 @@ static int run_pipeline(Plan& p, const void* in, const double* gl, const double*
             e = launch_fdm_tc_refine(fa, s);
         else
             e = launch_fdm_fast(prec, fa, s, rv & 1);
+    } else if (p.multi) {
+        MultiArgs ma{};
+        ma.spec = spec;
+        ma.elem_stride = p.elem_spec;
+        ma.P = N;
+        ma.n = p.n;
+        ma.Ns = p.Ns;
+        ma.nrows = (int)p.nrows;
+        ma.grp_of_row = p.d_grp_of_row;
+        ma.m1 = adjoint ? p.d_mm1_adj : p.d_mm1;
+        ma.m2 = adjoint ? p.d_mm2_adj : p.d_mm2;
+        ma.lam = p.d_lam;
+        ma.sigma = p.d_sigma;
+        ma.hom = p.d_hom;
+        ma.homs = p.d_homs;
+        ma.itf = p.d_itf;
+        ma.d0 = p.d_d0;
+        ma.dN = p.d_dN;
+        ma.al = p.bc.alphal;
+        ma.ar = p.bc.alphar;
+        ma.periodic = p.periodic ? 1 : 0;
+        ma.adjoint = adjoint ? 1 : 0;
+        e = launch_multi(p.precision != HELM_FP32, ma, s);
     } else {
         e = launch_rows(p.method, prec, r, s);
     }
@@ -1789,7 +1827,7 @@ const char* helm_plan_kernels(helm_plan_t plan)
         const bool slab = rv == 2 && p.slab_ok && p.fast && p.precision != HELM_FP32;
         std::string rows;
         if (p.fd) rows = p.N <= 512 ? "thomas_warp_kernel" : "thomas_kernel";
-        else if (!p.fast) rows = "rows_kernel";
+        else if (!p.fast) rows = p.multi ? "multi_rows_kernel" : "rows_kernel";
         else if (slab) rows = "slab_kernel";
         else if ((p.precision == HELM_FP64 || rv == 3) && p.d_fmma) rows = (rv == 3 || rv == 0) ? "fdm_mma16_kernel" : "fdm_mma_kernel";
         else if (p.precision == HELM_FP32_REFINE && p.d_ftc && p.sweeps == 1 && rv == 0) rows = "fdm_tc_refine_kernel";

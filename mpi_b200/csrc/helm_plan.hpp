@@ -87,6 +87,14 @@ struct Plan {
     double* d_feN = nullptr;
     double* d_fc0 = nullptr;       // folded D2[int][0], D2[int][N-1]
     double* d_fcN = nullptr;
+    // several GLL elements, FDM method (helm_multi.cu): the two transforms in
+    // fragment order (forward, transposed) and the interface system's factors
+    bool multi = false;
+    double* d_mm1 = nullptr;
+    double* d_mm2 = nullptr;
+    double* d_mm1_adj = nullptr;
+    double* d_mm2_adj = nullptr;
+    double* d_itf = nullptr;
     // batched independent 2D problems of one size class (helm_batch_*): their
     // lambdas, and the element offsets of each problem in the caller's packed
     // f / u buffers
@@ -121,7 +129,7 @@ struct Plan {
     bool eig_ok = false;           // its data are on the device
     double* d_hbc = nullptr;       // [4][32] first transform of the folded boundary columns
     double* d_frecip64 = nullptr;  // FP64 reciprocal shifts (refined plans; FP64 plans use d_frecip)
-    int* d_grp_of_row = nullptr;   // shift group of each spectrum row (slab kernel)
+    int* d_grp_of_row = nullptr;   // shift group of each spectrum row (slab, eigen-basis, several-element kernels)
     // device status word of the eigen-basis pipeline's TMA loads: a bounded wait
     // that ran out sets it to a nonzero code (helm_plan_device_status)
     int* d_status = nullptr;
