@@ -1,4 +1,4 @@
-// Kernel argument blocks shared by the launchers (helm_kernels.cu) and the plan
+// Kernel argument blocks shared by the launchers (helm_fft.cu, helm_kernels.cu) and the plan
 // (helm_plan.cu).
 #pragma once
 #include <cstdint>
@@ -68,6 +68,9 @@ struct FftArgs {
     // C2R only (forward): add the result to out instead of storing it (the
     // correction of a refinement sweep accumulated into the solution)
     int accumulate;
+    // set by launch_fft: bit 0 / bit 1, the column pairs of the input / output
+    // are aligned to their size, so a pair moves as one access
+    int pair;
 };
 
 // Finite-difference variant: one tridiagonal solve along z per spectrum row.
@@ -143,7 +146,7 @@ struct GllDerivArgs {
 };
 int launch_gll_deriv(int io_double, const GllDerivArgs& a, cudaStream_t s);
 
-// Launchers (helm_kernels.cu).  Return a cudaError_t.
+// Launchers (helm_fft.cu, helm_kernels.cu).  Return a cudaError_t.
 // T: compute precision (0 = float, 1 = double); io: real element bytes for
 // R2C input / C2R output (4 or 8).
 // variant: launch shape chosen by the plan's autotuner (0: 256-thread CTAs, 1: 128).
