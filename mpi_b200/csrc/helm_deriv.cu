@@ -507,7 +507,7 @@ static int run_gll_deriv_bulk(const GllDerivArgs& a, cudaStream_t s)
     if (stages < 2) return -1;  // not this kernel
     const size_t smem = L.b_bytes + (size_t)stages * (tile_bytes + sizeof(uint64_t));
     auto k = gll_deriv_bulk_kernel<NT>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(k, smem);
     if (e != cudaSuccess) return (int)e;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
@@ -534,15 +534,12 @@ static int run_gll_deriv_mma(const GllDerivArgs& a, cudaStream_t s)
     if (warps < 1) return (int)cudaErrorInvalidValue;
     const size_t smem = L.b_bytes + (size_t)warps * L.warp_bytes;
     auto k = gll_deriv_mma_kernel<NT>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(k, smem);
     if (e != cudaSuccess) return (int)e;
-    int dev = 0, sms = 148, per = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, warps * 32, smem);
-    if (per < 1) per = 1;
+    static std::atomic<unsigned long long> memo{0};
+    const long long resident = resident_ctas(k, warps * 32, smem, memo);
     const long long tiles = (a.nrows + GM_ROWS - 1) / GM_ROWS;
-    long long grid = (long long)sms * per;
+    long long grid = resident;
     if (grid > tiles) grid = tiles;
     if (grid < 1) return 0;
     return (int)launch_k(k, dim3((unsigned)grid), dim3(warps * 32), smem, s, a, L);
@@ -593,15 +590,12 @@ static int run_gll_deriv(const GllDerivArgs& a, cudaStream_t s)
     if (warps < 1) return (int)cudaErrorInvalidValue;
     const size_t smem = L.ef_bytes + (size_t)warps * L.warp_bytes;
     auto k = gll_deriv_kernel<T>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(k, smem);
     if (e != cudaSuccess) return (int)e;
-    int dev = 0, sms = 148, per = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, warps * 32, smem);
-    if (per < 1) per = 1;
+    static std::atomic<unsigned long long> memo{0};
+    const long long resident = resident_ctas(k, warps * 32, smem, memo);
     const long long tiles = (a.nrows + 31) / 32;
-    long long grid = (long long)sms * per;
+    long long grid = resident;
     if (grid > tiles) grid = tiles;
     if (grid < 1) return 0;
     return (int)launch_k(k, dim3((unsigned)grid), dim3(warps * 32), smem, s, a, L);

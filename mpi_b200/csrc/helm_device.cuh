@@ -2,6 +2,7 @@
 // float2/double2, in-register power-of-2 DFTs, and one Stockham pass of a
 // batched strided-axis FFT held in shared memory.
 #pragma once
+#include <atomic>
 #include <cstdlib>
 #include <cuda_runtime.h>
 #include <cstdint>
@@ -281,6 +282,34 @@ inline bool pdl_enabled()
         return !(e && e[0] == '0');
     }();
     return on;
+}
+
+// Host side: allow `k` its dynamic shared memory.  The default limit (48 KB with
+// the kernel's static arrays) needs no call, and a call is a third of a launch's
+// host time; launches are what a small solve costs on the host.
+template <typename K>
+inline cudaError_t allow_smem(K k, size_t smem)
+{
+    if (smem <= 40 * 1024) return cudaSuccess;
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+}
+
+// Host side: CTAs of `k` the current device holds at once, the grid of a
+// persistent kernel.  `memo` (one per kernel, static at the caller) holds the
+// last answer with the question it belongs to: the query costs more than a launch.
+template <typename K>
+inline long long resident_ctas(K k, int threads, size_t smem, std::atomic<unsigned long long>& memo)
+{
+    int dev = 0, sms = 148, per = 1;
+    cudaGetDevice(&dev);
+    const unsigned long long key = ((unsigned long long)smem << 24) | ((unsigned long long)threads << 8) | (unsigned)dev;
+    const unsigned long long m = memo.load(std::memory_order_relaxed);
+    if (m >> 16 == (key & 0xffffffffffffULL) && dev < 256) return (long long)(m & 0xffff);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, threads, smem);
+    const long long n = (long long)sms * (per < 1 ? 1 : per);
+    if (n < 65536 && dev < 256) memo.store((key << 16) | (unsigned long long)n, std::memory_order_relaxed);
+    return n;
 }
 
 template <typename... KArgs, typename... Args>

@@ -779,7 +779,7 @@ __global__ void __launch_bounds__(EpShape<L>::THREADS, 1) eig_solve2d_kernel(Eig
 template <typename K>
 cudaError_t prep(K k, size_t smem)
 {
-    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return allow_smem(k, smem);
 }
 
 template <int L>

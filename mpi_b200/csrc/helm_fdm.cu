@@ -438,16 +438,13 @@ static int run_fdm(const FdmArgs& a, cudaStream_t s)
 {
     auto k = fdm_fast_kernel<TS, TF, NSS, RPW, REFINE, ADJ>;
     const FdmSmem L = fdm_smem_layout<TS, TF, REFINE, RPW>(a.ld);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total);
+    cudaError_t e = allow_smem(k, L.total);
     if (e != cudaSuccess) return (int)e;
-    int dev = 0, sms = 148, per = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, FDM_WARPS * 32, L.total);
-    if (per < 1) per = 1;
+    static std::atomic<unsigned long long> memo{0};
+    const long long resident = resident_ctas(k, FDM_WARPS * 32, L.total, memo);
     const long long packs = (a.nrows + RPW - 1) / RPW;
     long long grid = (packs + FDM_WARPS - 1) / FDM_WARPS;
-    if (grid > (long long)sms * per) grid = (long long)sms * per;
+    if (grid > resident) grid = resident;
     if (grid <= 0) return 0;
     return (int)launch_k(k, dim3((unsigned)grid), dim3(FDM_WARPS * 32), L.total, s, a);
 }
@@ -708,16 +705,13 @@ static int run_fdm_mma(const FdmArgs& a, cudaStream_t s)
 {
     using S = MmaShape<NSS, NT, WARPS>;
     auto k = fdm_mma_kernel<NSS, NT, WARPS, ADJ>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem);
+    cudaError_t e = allow_smem(k, S::smem);
     if (e != cudaSuccess) return (int)e;
-    int dev = 0, sms = 148, per = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, WARPS * 32, S::smem);
-    if (per < 1) per = 1;
+    static std::atomic<unsigned long long> memo{0};
+    const long long resident = resident_ctas(k, WARPS * 32, S::smem, memo);
     const long long packs = (a.nrows + S::RPW - 1) / S::RPW;
     long long grid = (packs + WARPS - 1) / WARPS;
-    if (grid > (long long)sms * per) grid = (long long)sms * per;
+    if (grid > resident) grid = resident;
     if (grid <= 0) return 0;
     return (int)launch_k(k, dim3((unsigned)grid), dim3(WARPS * 32), S::smem, s, a);
 }
@@ -898,16 +892,13 @@ static int run_fdm_mma16(const FdmArgs& a, cudaStream_t s)
 {
     using S = MmaShape<NSS, 1, WARPS>;
     auto k = fdm_mma16_kernel<NSS, WARPS, ADJ>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem);
+    cudaError_t e = allow_smem(k, S::smem);
     if (e != cudaSuccess) return (int)e;
-    int dev = 0, sms = 148, per = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, WARPS * 32, S::smem);
-    if (per < 1) per = 1;
+    static std::atomic<unsigned long long> memo{0};
+    const long long resident = resident_ctas(k, WARPS * 32, S::smem, memo);
     const long long packs = (a.nrows + S::RPW - 1) / S::RPW;
     long long grid = (packs + WARPS - 1) / WARPS;
-    if (grid > (long long)sms * per) grid = (long long)sms * per;
+    if (grid > resident) grid = resident;
     if (grid <= 0) return 0;
     return (int)launch_k(k, dim3((unsigned)grid), dim3(WARPS * 32), S::smem, s, a);
 }
@@ -1065,7 +1056,7 @@ static int run_slab(const FdmArgs& a, const SlabArgs& sa, int nkx, cudaStream_t 
 {
     auto k = a.adjoint ? slab_kernel<L, true> : slab_kernel<L, false>;
     const size_t smem = slab_smem_bytes(L, sa.HS);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(k, smem);
     if (e != cudaSuccess) return (int)e;
     return (int)launch_k(k, dim3(2 * nkx), dim3(SLAB_WARPS * 32), smem, s, a, sa);
 }
@@ -1405,16 +1396,13 @@ int launch_fdm_tc_refine(const FdmArgs& a, cudaStream_t s)
 {
     if (a.ld != TC_LD || !a.tc_mats || !a.tc_m || a.sweeps != 1) return (int)cudaErrorInvalidValue;
     auto k = a.adjoint ? fdm_tc_refine_kernel<true> : fdm_tc_refine_kernel<false>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TC_SMEM);
+    cudaError_t e = allow_smem(k, TC_SMEM);
     if (e != cudaSuccess) return (int)e;
-    int dev = 0, sms = 148, per = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, TC_WARPS * 32, TC_SMEM);
-    if (per < 1) per = 1;
+    static std::atomic<unsigned long long> memo{0};
+    const long long resident = resident_ctas(k, TC_WARPS * 32, TC_SMEM, memo);
     const long long packs = (a.nrows + 3) / 4;
     long long grid = (packs + TC_WARPS - 1) / TC_WARPS;
-    if (grid > (long long)sms * per) grid = (long long)sms * per;
+    if (grid > resident) grid = resident;
     if (grid <= 0) return 0;
     return (int)launch_k(k, dim3((unsigned)grid), dim3(TC_WARPS * 32), TC_SMEM, s, a);
 }

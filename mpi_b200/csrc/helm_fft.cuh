@@ -857,16 +857,12 @@ static int run_fft_pipe(const FftArgs& a, long long total_cols, cudaStream_t s)
     using PS = PipeShape<T, TIO, L, THREADS, SMALL>;
     auto k = fft_pipe_kernel<T, TIO, L, DIR, MODE, THREADS, SMALL>;
     if (PS::smem > kMaxSmemPerBlock) return (int)cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PS::smem);
+    cudaError_t e = allow_smem(k, PS::smem);
     if (e != cudaSuccess) return (int)e;
     const long long tiles = (total_cols + S::CT - 1) / S::CT;
     if (tiles <= 0) return 0;
-    int dev = 0, sms = 148, per = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, THREADS, PS::smem);
-    if (per < 1) per = 1;
-    long long grid = (long long)sms * per;
+    static std::atomic<unsigned long long> memo{0};
+    long long grid = resident_ctas(k, THREADS, PS::smem, memo);
     if (grid > tiles) grid = tiles;
     return (int)launch_k(k, dim3((unsigned)grid), dim3(THREADS), PS::smem, s, a, total_cols, tiles);
 }
@@ -876,7 +872,7 @@ static int run_fft(const FftArgs& a, long long total_cols, cudaStream_t s)
 {
     using S = FftShape<T, L, THREADS, SMALL>;
     auto k = fft_kernel<T, TIO, L, DIR, MODE, THREADS, SMALL>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem);
+    cudaError_t e = allow_smem(k, S::smem);
     if (e != cudaSuccess) return (int)e;
     const long long blocks = (total_cols + S::CT - 1) / S::CT;
     if (blocks <= 0) return 0;

@@ -5,6 +5,8 @@
 //     the Robin ends (NonPeriodic2D_MPI.cpp:265-295, 414-424) and the combination
 //     u = phi + zl ul + zr ur (:466-470), fused, one warp per complex row (the LU
 //     method; fast-diagonalisation plans with several elements: helm_multi.cu).
+#include <algorithm>
+
 #include "helm_device.cuh"
 #include "helm_kernels.cuh"
 
@@ -540,16 +542,13 @@ static int run_rows(const RowArgs& a, cudaStream_t s)
 {
     auto k = rows_kernel<TS, TF, NSLOT, METHOD, REFINE, ADJ>;
     const RowSmem L = row_smem_layout<TS, TF, METHOD, REFINE>(a.n, a.ldf);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.total);
+    cudaError_t e = allow_smem(k, L.total);
     if (e != cudaSuccess) return (int)e;
     int grid = a.ngroups;
     if (METHOD == 2) {
-        int dev = 0, sms = 148, per = 1;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, ROW_WARPS * 32, L.total);
-        if (per < 1) per = 1;
-        grid = a.ngroups < sms * per ? a.ngroups : sms * per;
+        static std::atomic<unsigned long long> memo{0};
+        const long long resident = resident_ctas(k, ROW_WARPS * 32, L.total, memo);
+        grid = (int)std::min<long long>(a.ngroups, resident);
     }
     if (grid <= 0) return 0;
     return (int)launch_k(k, dim3(grid), dim3(ROW_WARPS * 32), L.total, s, a);
@@ -857,16 +856,13 @@ static int run_thomas_warp(const ThomasArgs& a, cudaStream_t s)
 {
     auto k = thomas_warp_kernel<T, M, LPR>;
     const size_t smem = (size_t)TRI_WARPS * 2 * (32 / LPR) * LPR * (M + 1) * sizeof(cplx_t<T>);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(k, smem);
     if (e != cudaSuccess) return (int)e;
-    int dev = 0, sms = 148, per = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, TRI_WARPS * 32, smem);
-    if (per < 1) per = 1;
+    static std::atomic<unsigned long long> memo{0};
+    const long long resident = resident_ctas(k, TRI_WARPS * 32, smem, memo);
     const long long rows_per_cta = (long long)TRI_WARPS * (32 / LPR);
     long long grid = (a.nrows + rows_per_cta - 1) / rows_per_cta;
-    if (grid > (long long)sms * per) grid = (long long)sms * per;
+    if (grid > resident) grid = resident;
     if (grid <= 0) return 0;
     return (int)launch_k(k, dim3((unsigned)grid), dim3(TRI_WARPS * 32), smem, s, a);
 }

@@ -325,7 +325,7 @@ int run_multi(MultiArgs a, cudaStream_t s)
     a.rows_per_cta = R;
     const size_t smem = multi_smem<TS>(R, a.Ns, a.P, a.n).total;
     if (smem > kMaxSmemPerBlock) return (int)cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(k, smem);
     if (e != cudaSuccess) return (int)e;
     const int tasks = (R * a.Ns + 3) / 4;
     const int threads = tasks >= 5 ? 256 : tasks >= 3 ? 128 : 64;
