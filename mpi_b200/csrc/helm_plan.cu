@@ -761,12 +761,13 @@ static int fft_pass(Plan& p, int L, int mode, int dir, const void* in, void* out
     const int kmode = a.adj_mode ? (int)FFT_C2R_ADJ : mode;
     // Spectral derivatives take their own launch shape: the solve's variant of
     // the same stage is tuned for another kernel (on eigen-basis plans the
-    // stage-1 bits select the y-convolution pass).  Unless pinned: 512-thread
-    // CTAs from length 512; below, the radix-8 schedule, in the persistent
-    // pipelined kernel for FP32 transforms.  Measured at 256^2 x 65 (FP64 I/O):
-    // FP64 d/dx 33.8 us (radix-16 shapes 44.0, pipelined 37.9), FP32 31.7 us
-    // (plain 33.8); at 512^2 x 33 FP64 d/dx 62.4 us (256 threads 76.7).
-    const int dvar = p.deriv_var >= 0 ? p.deriv_var : (L >= 512 ? 8 : td ? 2 : 6);
+    // stage-1 bits select the y-convolution pass).  Unless pinned, with arrays
+    // beyond L2 (FP64, x / y, us): y passes, whose odd row strides leave the pairs
+    // split, on the radix-8 schedule where there is one (256 x 256 x 65: y 27.6,
+    // radix 16 38.5); FP64 x passes up to 256 on 128-thread CTAs of radix 16
+    // (20.3; 256 threads 22.8, radix 8 24.0); the rest on 256 threads (512 x 128 x
+    // 65: x 29.7, 512-thread CTAs 35.2; FP32 256 x 256 x 65: x 14.1, radix 8 16.5).
+    const int dvar = p.deriv_var >= 0 ? p.deriv_var : stage == 1 ? 2 : (td && L <= 256) ? 1 : 0;
     const int var = mode == FFT_DERIV ? dvar : sub ? (p.fft_var[stage] & ~4) : p.fft_var[stage];
     int e = launch_fft(L, kmode, dir, td, io, a, ccols * nbatch, s, var);
     if (e) return set_cuda_error((cudaError_t)e, "fft launch");
