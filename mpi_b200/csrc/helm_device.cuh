@@ -32,6 +32,41 @@ template <typename C> __device__ __forceinline__ C cmulc(C a, C b)
     return mk(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
 }
 
+// Two neighbouring values as one access of twice their size, to whose multiple p
+// is aligned (32 bytes for complex doubles).
+__device__ __forceinline__ void ld_pair(const float* p, float& a, float& b)
+{
+    const float2 v = *reinterpret_cast<const float2*>(p);
+    a = v.x; b = v.y;
+}
+__device__ __forceinline__ void ld_pair(const double* p, double& a, double& b)
+{
+    const double2 v = *reinterpret_cast<const double2*>(p);
+    a = v.x; b = v.y;
+}
+__device__ __forceinline__ void st_pair(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
+__device__ __forceinline__ void st_pair(double* p, double a, double b)
+{
+    *reinterpret_cast<double2*>(p) = make_double2(a, b);
+}
+__device__ __forceinline__ void ld_pair(const float2* p, float2& a, float2& b)
+{
+    const float4 v = *reinterpret_cast<const float4*>(p);
+    a = mk(v.x, v.y); b = mk(v.z, v.w);
+}
+__device__ __forceinline__ void ld_pair(const double2* p, double2& a, double2& b)
+{
+    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];\n" : "=d"(a.x), "=d"(a.y), "=d"(b.x), "=d"(b.y) : "l"(p) : "memory");
+}
+__device__ __forceinline__ void st_pair(float2* p, float2 a, float2 b)
+{
+    *reinterpret_cast<float4*>(p) = make_float4(a.x, a.y, b.x, b.y);
+}
+__device__ __forceinline__ void st_pair(double2* p, double2 a, double2 b)
+{
+    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};\n" ::"l"(p), "d"(a.x), "d"(a.y), "d"(b.x), "d"(b.y) : "memory");
+}
+
 // cos and sin of 2*pi*m/16 for m = 0..7 (exact constants of the 16th roots of unity).
 __device__ __forceinline__ double root16_cos(int m)
 {
@@ -108,6 +143,65 @@ template <int L, int SMALL> struct RadixV : Radix<L> {};
 template <> struct RadixV<128, 1> { static constexpr int n = 3, r0 = 8, r1 = 4, r2 = 4; };
 template <> struct RadixV<256, 1> { static constexpr int n = 3, r0 = 8, r1 = 8, r2 = 4; };
 template <int L> constexpr bool has_small_radix() { return L == 128 || L == 256; }
+
+// The inverse of a length-L forward transform whose last pass has left its outputs
+// in registers (item (t, r) of radix RL at row tc + t TPC + r L / RL): the same
+// passes backwards, each radix-R butterfly before its conjugated twiddles.  No
+// reordering pass between the two transforms, as an inverse in the forward's own
+// order would need: one exchange fewer through shared memory.  sm: the exchange
+// buffer [L][hs], column cl; on return v[r] holds row tc + r TPC, unscaled.  All
+// threads of the CTA call it; the first write goes to the rows this thread read
+// last, so it needs no barrier before it.
+template <int R, int NS, int TPC, int L, int R0, typename T>
+__device__ __forceinline__ void mirror_pass(const cplx_t<T>* tw, int tc, cplx_t<T> (&v)[R0])
+{
+#pragma unroll
+    for (int t = 0; t < R0 / R; ++t) {
+        cplx_t<T> w[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) w[r] = v[t * R + r];
+        dft_reg<R, 1, T>(w);
+        const int jm = (tc + t * TPC) % NS;
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[t * R + r] = r ? cmulc(w[r], tw[r * jm * (L / (NS * R))]) : w[r];
+    }
+}
+
+template <typename T, int L, int TPC, int R0, int R1, int R2, int NP>
+__device__ __forceinline__ void fft_inverse_mirror(cplx_t<T>* sm, int hs, const cplx_t<T>* tw, int tc, int cl,
+                                                   cplx_t<T> (&v)[R0])
+{
+    // the twiddles are the forward's: without this the compiler holds them in
+    // registers from one transform to the other, and spills
+    asm volatile("" : "+l"(tw));
+    if constexpr (NP == 3) {
+        mirror_pass<R2, R0 * R1, TPC, L, R0, T>(tw, tc, v);
+#pragma unroll
+        for (int t = 0; t < R0 / R2; ++t)
+#pragma unroll
+            for (int r = 0; r < R2; ++r) sm[(tc + t * TPC + r * (L / R2)) * hs + cl] = v[t * R2 + r];
+        __syncthreads();
+#pragma unroll
+        for (int t = 0; t < R0 / R1; ++t)
+#pragma unroll
+            for (int r = 0; r < R1; ++r) {
+                const int j = tc + t * TPC;
+                v[t * R1 + r] = sm[((j / R0) * R0 * R1 + j % R0 + r * R0) * hs + cl];
+            }
+        __syncthreads();
+    }
+    if constexpr (NP >= 2) {
+        mirror_pass<R1, R0, TPC, L, R0, T>(tw, tc, v);
+#pragma unroll
+        for (int t = 0; t < R0 / R1; ++t)
+#pragma unroll
+            for (int r = 0; r < R1; ++r) sm[(tc + t * TPC + r * (L / R1)) * hs + cl] = v[t * R1 + r];
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < R0; ++r) v[r] = sm[(tc * R0 + r) * hs + cl];
+    }
+    dft_reg<R0, 1, T>(v);
+}
 
 // ---- FFT of columns held in shared memory (slab and eigen-basis kernels) ----
 

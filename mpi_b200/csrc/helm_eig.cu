@@ -30,6 +30,7 @@
 
 #include <cooperative_groups.h>
 #include <cstring>
+#include <type_traits>
 
 namespace cg = cooperative_groups;
 
@@ -343,54 +344,78 @@ __global__ void __launch_bounds__(EpShape<L>::THREADS, 1) eig_fwd_kernel(EigArgs
     double2* Sg = reinterpret_cast<double2*>(a.S);
     const long long Ny = a.Ny;
     r2c_split<L>(z, warp, lane, [&](int kx, int c, double2 X, double2 Y) {
-        double2* row = Sg + ((long long)kx * Ny + y) * EIG_SLOTS;
-        row[2 * c] = X;
-        row[2 * c + 1] = Y;
+        st_pair(Sg + ((long long)kx * Ny + y) * EIG_SLOTS + 2 * c, X, Y);
     });
 }
 
 // ------------------------------------------------------------------ pass 2 --
-// CTA shapes of pass 2: 16 coefficient columns per tile and 256 threads (two
-// CTAs per SM), or 8 columns and 128 threads (four per SM, more tiles in
-// flight); launch variant bit 0 of the y pass picks one.
-template <int NY, int CT, int THREADS>
-__global__ void __launch_bounds__(THREADS, 512 / THREADS) eig_conv_kernel(EigArgs a)
+// Forward FFT along y, scaling, inverse FFT of CT coefficient columns of one kx, a
+// thread's radix-R0 share of one column in registers throughout: the inverse runs
+// the forward's passes backwards (fft_inverse_mirror), so a value passes through
+// shared memory twice (four times for Ny = 512) instead of six times.  Bound: the
+// FP64 pipe and the 2 x 33.8 MB of spectrum (256 x 256 modes, mostly in L2).  From
+// pass start to pass start 36.4 -> 28.9 us there; with the pairs of spectrum values
+// stored and loaded as one access in passes 1 and 3 (36.1 -> 32.7 and 34.6 -> 34.1
+// us) the solve of 256 x 256 x 65 went from 91.5 to 79.9 us.  CTAs of 256 or of 128
+// threads (half the columns, more tiles in flight): launch variant bit 0 of the y
+// pass; short transforms use as many threads as 64 columns have work for.
+template <int NY>
+struct ConvShape {
+    using RS = typename std::conditional<NY == 512, Radix512Wide, Radix<NY>>::type;
+    static constexpr int TPC = NY / RS::r0;  // threads per column
+};
+template <int NY, int THREADS>
+constexpr int conv_cols()
 {
+    return THREADS / ConvShape<NY>::TPC < EIG_SLOTS ? THREADS / ConvShape<NY>::TPC : EIG_SLOTS;
+}
+
+template <int NY, int CT>
+__global__ void __launch_bounds__(CT * ConvShape<NY>::TPC, 512 / (CT * ConvShape<NY>::TPC)) eig_conv_kernel(EigArgs a)
+{
+    using RS = typename ConvShape<NY>::RS;
+    constexpr int TPC = ConvShape<NY>::TPC, R0 = RS::r0, R1 = RS::r1, R2 = RS::r2, NP = RS::n;
+    constexpr int RL = NP == 1 ? R0 : NP == 2 ? R1 : R2;  // radix of the last pass
     extern __shared__ __align__(16) double esm[];
     double2* sm = reinterpret_cast<double2*>(esm);
     constexpr int TILES = EIG_SLOTS / CT;
     const int kx = blockIdx.x / TILES, j0 = (blockIdx.x - kx * TILES) * CT;
-    double2* Sg = reinterpret_cast<double2*>(a.S) + (long long)kx * NY * EIG_SLOTS + j0;
-    pdl_enter();
-    for (int e = threadIdx.x; e < NY * CT; e += blockDim.x) {
-        const int ky = e / CT, c = e - ky * CT;
-        cp_async_bytes16(&sm[ky * CT + c], &Sg[(long long)ky * EIG_SLOTS + c], true);
-    }
-    cp_async_commit();
-    // this thread's scale factors, fetched while the tile is in flight
-    constexpr int PER = (NY * CT + THREADS - 1) / THREADS;
-    double r[PER];
-    const double* rc = a.recip;
-#pragma unroll
-    for (int k = 0; k < PER; ++k) {
-        const int e = threadIdx.x + THREADS * k, ky = e / CT, c = e - ky * CT;
-        r[k] = e < NY * CT ? rc[(long long)a.grp_of_row[kx * NY + ky] * EIG_SLOTS + j0 + c] * a.scale : 0.0;
-    }
-    cp_async_wait_all();
-    __syncthreads();
+    const int tc = threadIdx.x / CT, cl = threadIdx.x - tc * CT;
+    double2* col = reinterpret_cast<double2*>(a.S) + (long long)kx * NY * EIG_SLOTS + j0 + cl;
     const double2* tw = static_cast<const double2*>(a.tw_y);
-    slab_fft<NY, -1, THREADS>(sm, CT, CT, tw);
+    const int* grp = a.grp_of_row + kx * NY;
+    const double* rc = a.recip + j0 + cl;
+    pdl_enter();
+    double2 v[R0];
 #pragma unroll
-    for (int k = 0; k < PER; ++k) {
-        const int e = threadIdx.x + THREADS * k;
-        if (e < NY * CT) sm[e] = make_double2(sm[e].x * r[k], sm[e].y * r[k]);
+    for (int r = 0; r < R0; ++r) v[r] = col[(tc + r * TPC) * EIG_SLOTS];
+    dft_reg<R0, -1, double>(v);
+    if constexpr (NP >= 2) slab_to_smem<NY, R0, 1, TPC, R0>(sm, CT, tc, cl, v);
+    // the scale factors of this thread's last-pass rows, on their way while the
+    // passes between run
+    double sc[R0];
+#pragma unroll
+    for (int t = 0; t < R0 / RL; ++t)
+#pragma unroll
+        for (int r = 0; r < RL; ++r) sc[t * RL + r] = rc[(long long)grp[tc + t * TPC + r * (NY / RL)] * EIG_SLOTS];
+    if constexpr (NP >= 2) {
+        __syncthreads();
+        slab_from_smem<NY, R1, R0, -1, TPC, R0>(sm, CT, tw, tc, cl, v);
     }
-    __syncthreads();
-    slab_fft<NY, 1, THREADS>(sm, CT, CT, tw);
-    for (int e = threadIdx.x; e < NY * CT; e += blockDim.x) {
-        const int ky = e / CT, c = e - ky * CT;
-        Sg[(long long)ky * EIG_SLOTS + c] = sm[ky * CT + c];
+    if constexpr (NP >= 3) {
+        __syncthreads();
+        slab_to_smem<NY, R1, R0, TPC, R0>(sm, CT, tc, cl, v);
+        __syncthreads();
+        slab_from_smem<NY, R2, R0 * R1, -1, TPC, R0>(sm, CT, tw, tc, cl, v);
     }
+#pragma unroll
+    for (int i = 0; i < R0; ++i) {
+        const double f = sc[i] * a.scale;
+        v[i] = make_double2(v[i].x * f, v[i].y * f);
+    }
+    fft_inverse_mirror<double, NY, TPC, R0, R1, R2, NP>(sm, CT, tw, tc, cl, v);
+#pragma unroll
+    for (int r = 0; r < R0; ++r) col[(tc + r * TPC) * EIG_SLOTS] = v[r];
 }
 
 // Adjoint: the boundary terms of the transposed map for the warp's rows,
@@ -498,9 +523,7 @@ __global__ void __launch_bounds__(EpShape<L>::THREADS, 1) eig_inv_kernel(EigArgs
     const long long Ny = a.Ny;
     pdl_enter();
     c2r_assemble<L>(z, warp, lane, [&](int kx, int c, double2& X, double2& Y) {
-        const double2* row = Sg + ((long long)kx * Ny + y) * EIG_SLOTS;
-        X = row[2 * c];
-        Y = row[2 * c + 1];
+        ld_pair(Sg + ((long long)kx * Ny + y) * EIG_SLOTS + 2 * c, X, Y);
     });
     __syncthreads();
     slab_fft<L, 1, S::THREADS>(z, EP_HS, 32, static_cast<const double2*>(a.tw_x));
@@ -644,9 +667,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SplitShape<L>::THREA
     for (int kp = warp; kp <= kmax; kp += S::WARPS) {
         const int km = rank == 0 ? ((H - kp) & (H - 1)) : (H - 1 - kp);
         const double2 zk = z[kp * EP_HS + lane], zm = z[km * EP_HS + lane];
-        double2* row = Sg + ((long long)(2 * kp + rank) * Ny + y) * EIG_SLOTS;
-        row[2 * lane] = make_double2(0.5 * (zk.x + zm.x), 0.5 * (zk.y - zm.y));
-        row[2 * lane + 1] = make_double2(0.5 * (zk.y + zm.y), 0.5 * (zm.x - zk.x));
+        st_pair(Sg + ((long long)(2 * kp + rank) * Ny + y) * EIG_SLOTS + 2 * lane,
+                make_double2(0.5 * (zk.x + zm.x), 0.5 * (zk.y - zm.y)),
+                make_double2(0.5 * (zk.y + zm.y), 0.5 * (zm.x - zk.x)));
     }
 }
 
@@ -676,9 +699,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SplitShape<L>::THREA
 #pragma unroll
         for (int b = 0; b < NB; ++b)
             if (k0 + b * W <= kmax) {
-                const double2* row = Sg + ((long long)(2 * (k0 + b * W) + rank) * Ny + y) * EIG_SLOTS;
-                X[b] = row[2 * lane];
-                Y[b] = row[2 * lane + 1];
+                ld_pair(Sg + ((long long)(2 * (k0 + b * W) + rank) * Ny + y) * EIG_SLOTS + 2 * lane, X[b], Y[b]);
             }
 #pragma unroll
         for (int b = 0; b < NB; ++b) {
@@ -827,25 +848,23 @@ int run_3d(int pass, const EigArgs& a, cudaStream_t s)
     const int nkx = L / 2 + 1;
     const bool narrow = a.conv_var & 1;
     switch (a.Ny) {
-#define HELM_EIG_CONV(NY, CT, TH)                                                                               \
-    {                                                                                                           \
-        const size_t sm2 = (size_t)NY * CT * sizeof(double2);                                                   \
-        if ((e = prep(eig_conv_kernel<NY, CT, TH>, sm2)) != cudaSuccess) return (int)e;                         \
-        return (int)launch_k(eig_conv_kernel<NY, CT, TH>, dim3(nkx * (EIG_SLOTS / CT)), dim3(TH), sm2, s, a);   \
+#define HELM_EIG_CONV(NY)                                                                              \
+    case NY: {                                                                                         \
+        constexpr int TPC = ConvShape<NY>::TPC, W = conv_cols<NY, 256>(), H = conv_cols<NY, 128>();    \
+        const int ct = narrow ? H : W;                                                                 \
+        auto k = narrow ? eig_conv_kernel<NY, H> : eig_conv_kernel<NY, W>;                             \
+        const size_t sm2 = (size_t)NY * ct * sizeof(double2);                                          \
+        if ((e = prep(k, sm2)) != cudaSuccess) return (int)e;                                          \
+        return (int)launch_k(k, dim3(nkx * (EIG_SLOTS / ct)), dim3(ct * TPC), sm2, s, a);              \
     }
-#define HELM_EIG_CONV2(NY)                                                                                      \
-    case NY:                                                                                                    \
-        if (narrow) HELM_EIG_CONV(NY, 8, 128) else HELM_EIG_CONV(NY, 16, 256)
-        HELM_EIG_CONV2(4)
-        HELM_EIG_CONV2(8)
-        HELM_EIG_CONV2(16)
-        HELM_EIG_CONV2(32)
-        HELM_EIG_CONV2(64)
-        HELM_EIG_CONV2(128)
-        HELM_EIG_CONV2(256)
-        case 512:
-            if (narrow) HELM_EIG_CONV(512, 4, 256) else HELM_EIG_CONV(512, 8, 256)
-#undef HELM_EIG_CONV2
+        HELM_EIG_CONV(4)
+        HELM_EIG_CONV(8)
+        HELM_EIG_CONV(16)
+        HELM_EIG_CONV(32)
+        HELM_EIG_CONV(64)
+        HELM_EIG_CONV(128)
+        HELM_EIG_CONV(256)
+        HELM_EIG_CONV(512)
 #undef HELM_EIG_CONV
         default: return (int)cudaErrorInvalidValue;
     }

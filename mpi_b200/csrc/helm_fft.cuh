@@ -15,6 +15,16 @@ int launch_fft_f64(int L, int variant, int mode, int dir, const FftArgs& a, long
 int launch_fft_f32(int L, int variant, int mode, int dir, const FftArgs& a, long long total_cols, cudaStream_t s);
 int launch_fft_f32_f64(int L, int variant, int mode, int dir, const FftArgs& a, long long total_cols, cudaStream_t s);
 
+// The two neighbouring real columns of an R2C / C2R pair, or their two complex
+// spectrum values, as one access (ld_pair, st_pair; FftArgs::pair says that the addresses allow
+// it).  A thread that loads or stores the two separately leaves every other
+// 8 or 16 bytes to the next instruction: each of the two touches all sectors of
+// the row segment, and the stores reach L2 as partial sectors.  FP64 passes of
+// length 1024 over 1024 x 256 columns (a floor of 0.66 ms of HBM traffic):
+// real-to-complex 1.44 -> 1.13 ms, complex-to-real 1.71 -> 1.09 ms.  The choice
+// between pair and single accesses is made once around each unrolled loop: made
+// inside, every load waited for the one before.
+
 template <typename T, int L, int THREADS, int SMALL>
 struct FftShape {
     using RS = RadixV<L, SMALL>;
@@ -23,48 +33,6 @@ struct FftShape {
     static constexpr int CT = THREADS / TPC;    // columns per tile
     static constexpr size_t smem = (size_t)L * CT * sizeof(cplx_t<T>);
 };
-
-// The two neighbouring real columns of an R2C / C2R pair, or their two complex
-// spectrum values, as one access (FftArgs::pair says that the addresses allow
-// it).  A thread that loads or stores the two separately leaves every other
-// 8 or 16 bytes to the next instruction: each of the two touches all sectors of
-// the row segment, and the stores reach L2 as partial sectors.  FP64 passes of
-// length 1024 over 1024 x 256 columns (a floor of 0.66 ms of HBM traffic):
-// real-to-complex 1.44 -> 1.13 ms, complex-to-real 1.71 -> 1.09 ms.  The choice
-// between pair and single accesses is made once around each unrolled loop: made
-// inside, every load waited for the one before.
-__device__ __forceinline__ void ld_pair(const float* p, float& a, float& b)
-{
-    const float2 v = *reinterpret_cast<const float2*>(p);
-    a = v.x; b = v.y;
-}
-__device__ __forceinline__ void ld_pair(const double* p, double& a, double& b)
-{
-    const double2 v = *reinterpret_cast<const double2*>(p);
-    a = v.x; b = v.y;
-}
-__device__ __forceinline__ void st_pair(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
-__device__ __forceinline__ void st_pair(double* p, double a, double b)
-{
-    *reinterpret_cast<double2*>(p) = make_double2(a, b);
-}
-__device__ __forceinline__ void ld_pair(const float2* p, float2& a, float2& b)
-{
-    const float4 v = *reinterpret_cast<const float4*>(p);
-    a = mk(v.x, v.y); b = mk(v.z, v.w);
-}
-__device__ __forceinline__ void ld_pair(const double2* p, double2& a, double2& b)
-{
-    asm volatile("ld.global.v4.f64 {%0, %1, %2, %3}, [%4];\n" : "=d"(a.x), "=d"(a.y), "=d"(b.x), "=d"(b.y) : "l"(p) : "memory");
-}
-__device__ __forceinline__ void st_pair(float2* p, float2 a, float2 b)
-{
-    *reinterpret_cast<float4*>(p) = make_float4(a.x, a.y, b.x, b.y);
-}
-__device__ __forceinline__ void st_pair(double2* p, double2 a, double2 b)
-{
-    asm volatile("st.global.v4.f64 [%0], {%1, %2, %3, %4};\n" ::"l"(p), "d"(a.x), "d"(a.y), "d"(b.x), "d"(b.y) : "memory");
-}
 
 template <int R, int DIR, typename T>
 __device__ __forceinline__ void dft_sub(cplx_t<T>* v)
@@ -306,27 +274,6 @@ __device__ __forceinline__ cplx_t<T> deriv_mul_packed(int order, double w, int k
     return mk(m * Z.x, m * Z.y);
 }
 
-// Forward (DIR2 = -1) or inverse (+1) Stockham passes of a transform whose
-// first-pass inputs v[r] (rows tc + r TPC) are in registers; on return v holds
-// the outputs of the last pass (rows pass_out_row).
-template <typename T, int L, int DIR2, int TPC, int CT, int R0, int R1, int R2, int NP>
-__device__ __forceinline__ void fft_reg_passes(cplx_t<T>* sm, const cplx_t<T>* tw, int tc, int cl, cplx_t<T> (&v)[R0])
-{
-    dft_reg<R0, DIR2, T>(v);
-    if constexpr (NP >= 2) {
-        __syncthreads();
-        pass_to_smem<T, L, R0, 1, TPC, CT, R0>(sm, tc, cl, v);
-        __syncthreads();
-        pass_from_smem<T, L, R1, R0, DIR2, TPC, CT, R0>(sm, tw, tc, cl, v);
-    }
-    if constexpr (NP >= 3) {
-        __syncthreads();
-        pass_to_smem<T, L, R1, R0, TPC, CT, R0>(sm, tc, cl, v);
-        __syncthreads();
-        pass_from_smem<T, L, R2, R0 * R1, DIR2, TPC, CT, R0>(sm, tw, tc, cl, v);
-    }
-}
-
 // Warps an SM has room for: 24 (at most 85 registers a thread), or 16 where 16
 // points of 8 bytes a thread, or an adjoint pass's operands, would spill at that.
 template <typename T, typename TIO, int L, int MODE, int THREADS, int SMALL>
@@ -502,35 +449,27 @@ __global__ void __launch_bounds__(THREADS, (fft_min_ctas<T, TIO, L, MODE, THREAD
     // ---------------------------------------------------------- output --
     const T sc = (T)a.scale;
     if constexpr (MODE == FFT_DERIV) {
-        // multiply in place, back to natural row order through shared memory,
-        // then the inverse transform and the two real output columns
+        // multiply in place, inverse transform, the two real output columns
 #pragma unroll
         for (int t = 0; t < R0 / RL; ++t)
 #pragma unroll
             for (int r = 0; r < RL; ++r)
                 v[t * RL + r] = deriv_mul_packed<T, L>(a.deriv_order, a.deriv_w, pass_out_row<RL, NSL, TPC>(tc, t, r),
                                                        v[t * RL + r]);
-        __syncthreads();
-        pass_to_smem<T, L, RL, NSL, TPC, CT, R0>(sm, tc, cl, v);
-        __syncthreads();
-#pragma unroll
-        for (int r = 0; r < R0; ++r) v[r] = sm[(tc + r * TPC) * CT + cl];
-        fft_reg_passes<T, L, 1, TPC, CT, R0, R1, R2, NP>(sm, tw, tc, cl, v);
+        fft_inverse_mirror<T, L, TPC, R0, R1, R2, NP>(sm, CT, tw, tc, cl, v);
         if (valid) {
             TIO* out = static_cast<TIO*>(a.out) + out_base;
 #pragma unroll
-            for (int t = 0; t < R0 / RL; ++t)
-#pragma unroll
-                for (int r = 0; r < RL; ++r) {
-                    const long long row = pass_out_row<RL, NSL, TPC>(tc, t, r);
-                    const TIO x0 = (TIO)(v[t * RL + r].x * sc), x1 = (TIO)(v[t * RL + r].y * sc);
-                    if ((a.pair & 2) && has1) {
-                        st_pair(&out[row * a.out_row + c0], x0, x1);
-                    } else {
-                        out[row * a.out_row + c0] = x0;
-                        if (has1) out[row * a.out_row + c1] = x1;
-                    }
+            for (int r = 0; r < R0; ++r) {
+                const long long row = tc + r * TPC;
+                const TIO x0 = (TIO)(v[r].x * sc), x1 = (TIO)(v[r].y * sc);
+                if ((a.pair & 2) && has1) {
+                    st_pair(&out[row * a.out_row + c0], x0, x1);
+                } else {
+                    out[row * a.out_row + c0] = x0;
+                    if (has1) out[row * a.out_row + c1] = x1;
                 }
+            }
         }
     } else if constexpr (MODE == FFT_C2C) {
         if (valid) {
@@ -777,35 +716,27 @@ __global__ void __launch_bounds__(THREADS) fft_pipe_kernel(FftArgs a, long long 
         // ------------------------------------------------------ output --
         const T sc = (T)a.scale;
         if constexpr (MODE == FFT_DERIV) {
-            // multiplier in registers, natural row order through the tile's
-            // buffer, inverse transform, the two real output columns
+            // multiply in place, inverse transform, the two real output columns
 #pragma unroll
             for (int t = 0; t < R0 / RL; ++t)
 #pragma unroll
                 for (int r = 0; r < RL; ++r)
                     v[t * RL + r] = deriv_mul_packed<T, L>(a.deriv_order, a.deriv_w,
                                                            pass_out_row<RL, NSL, TPC>(tc, t, r), v[t * RL + r]);
-            __syncthreads();
-            pass_to_smem<T, L, RL, NSL, TPC, CT, R0>(sm, tc, cl, v);
-            __syncthreads();
-#pragma unroll
-            for (int r = 0; r < R0; ++r) v[r] = sm[(tc + r * TPC) * CT + cl];
-            fft_reg_passes<T, L, 1, TPC, CT, R0, R1, R2, NP>(sm, tw, tc, cl, v);
+            fft_inverse_mirror<T, L, TPC, R0, R1, R2, NP>(sm, CT, tw, tc, cl, v);
             if (valid) {
                 TIO* out = static_cast<TIO*>(a.out) + out_base;
 #pragma unroll
-                for (int t = 0; t < R0 / RL; ++t)
-#pragma unroll
-                    for (int r = 0; r < RL; ++r) {
-                        const long long row = pass_out_row<RL, NSL, TPC>(tc, t, r);
-                        const TIO x0 = (TIO)(v[t * RL + r].x * sc), x1 = (TIO)(v[t * RL + r].y * sc);
-                        if ((a.pair & 2) && has1) {
-                            st_pair(&out[row * a.out_row + c0], x0, x1);
-                        } else {
-                            out[row * a.out_row + c0] = x0;
-                            if (has1) out[row * a.out_row + c1] = x1;
-                        }
+                for (int r = 0; r < R0; ++r) {
+                    const long long row = tc + r * TPC;
+                    const TIO x0 = (TIO)(v[r].x * sc), x1 = (TIO)(v[r].y * sc);
+                    if ((a.pair & 2) && has1) {
+                        st_pair(&out[row * a.out_row + c0], x0, x1);
+                    } else {
+                        out[row * a.out_row + c0] = x0;
+                        if (has1) out[row * a.out_row + c1] = x1;
                     }
+                }
             }
         } else if constexpr (MODE == FFT_C2C) {
             if (valid) {

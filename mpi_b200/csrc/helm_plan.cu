@@ -763,10 +763,10 @@ static int fft_pass(Plan& p, int L, int mode, int dir, const void* in, void* out
     // the same stage is tuned for another kernel (on eigen-basis plans the
     // stage-1 bits select the y-convolution pass).  Unless pinned, with arrays
     // beyond L2 (FP64, x / y, us): y passes, whose odd row strides leave the pairs
-    // split, on the radix-8 schedule where there is one (256 x 256 x 65: y 27.6,
-    // radix 16 38.5); FP64 x passes up to 256 on 128-thread CTAs of radix 16
-    // (20.3; 256 threads 22.8, radix 8 24.0); the rest on 256 threads (512 x 128 x
-    // 65: x 29.7, 512-thread CTAs 35.2; FP32 256 x 256 x 65: x 14.1, radix 8 16.5).
+    // split, on the radix-8 schedule where there is one (256 x 256 x 65: y 25.8,
+    // radix 16 36.3); FP64 x passes up to 256 on 128-thread CTAs of radix 16
+    // (18.0; 256 threads 20.2, radix 8 22.1); the rest on 256 threads (512 x 128 x
+    // 65: x 27.6, 512-thread CTAs 33.2; FP32 256 x 256 x 65: x 13.1, radix 8 14.5).
     const int dvar = p.deriv_var >= 0 ? p.deriv_var : stage == 1 ? 2 : (td && L <= 256) ? 1 : 0;
     const int var = mode == FFT_DERIV ? dvar : sub ? (p.fft_var[stage] & ~4) : p.fft_var[stage];
     int e = launch_fft(L, kmode, dir, td, io, a, ccols * nbatch, s, var);
