@@ -28,14 +28,6 @@ namespace helm {
 
 constexpr int FDM_WARPS = 8;
 
-__device__ __forceinline__ float fshfl(float v, int s) { return __shfl_sync(0xffffffffu, v, s); }
-template <typename T> __device__ __forceinline__ T wsum(T v)
-{
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
 struct FdmSmem {
     size_t mats, d2, stage, total;
 };
@@ -140,9 +132,37 @@ __device__ __forceinline__ void fdm_folded_core(const TF* Ws, const TF* Vs, cons
     }
 }
 
+// Sums of NV values over the warp: every step halves the values a lane still
+// carries, so 16 sums take 16 shuffles instead of 80.  Sum i ends in the lanes
+// whose low log2(NV) bits are i with its bits reversed.
+template <typename T, int NV>
+__device__ __forceinline__ T warp_sums(T (&v)[NV], int lane)
+{
+    int o = 1;
+#pragma unroll
+    for (int nv = NV; nv > 1; nv >>= 1, o <<= 1) {
+        const bool up = lane & o;
+#pragma unroll
+        for (int i = 0; i < NV / 2; ++i)
+            if (i < nv / 2) {
+                const T send = up ? v[i] : v[i + nv / 2], keep = up ? v[i + nv / 2] : v[i];
+                v[i] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+            }
+    }
+#pragma unroll
+    for (int b = NV; b < 32; b <<= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], b);
+    return v[0];
+}
+
 // Epilogue of a folded solve for RPW rows: boundary values (Robin / interface
 // data, or the transposed 2x2 system of the adjoint), unfold, store.  x* hold
-// the folded solution, lane l owning fold index l + 32 t.
+// the folded solution, lane l owning fold index l + 32 t.  The boundary values of
+// the pack's rows are worked out side by side, one row's real or imaginary part a
+// lane, their operands fetched before the sums they wait for: a short grid runs
+// at the latency of one such chain, and row after row it was four of them.
+// With the plan data of a warp's first pack also fetched before the previous pass's
+// results are waited for, the row stage of 64 x 128 x 50 (Robin, FP64) went from
+// 17.3 to 14.4 us between events, 256 x 256 x 65 from 68 to 55 us (m8n8k4 63 to 51).
 template <typename TS, int NSS, int RPW, bool ADJ, typename RowOf>
 __device__ __forceinline__ void fdm_store_rows_at(const FdmArgs& a, RowOf row_of, const int (&grp)[RPW],
                                                   const bool (&ok)[RPW], const TS (&xsr)[RPW][NSS],
@@ -150,68 +170,92 @@ __device__ __forceinline__ void fdm_store_rows_at(const FdmArgs& a, RowOf row_of
                                                   const TS (&xdi)[RPW][NSS], int lane)
 {
     using CS = cplx_t<TS>;
+    constexpr int LOGV = RPW == 4 ? 4 : RPW == 2 ? 3 : 2;
     const int ld = a.ld, ms = a.ms, ma = a.ma, m = a.m, n = a.n, P = a.P;
     const TS r2 = (TS)0.70710678118654752440;
+    const bool bnd = a.hvec != nullptr;
+    // the interior correction zl hl + zr hr (skipped when hl = hr = 0: the
+    // transposed system of Dirichlet ends)
+    const bool hadd = bnd && !a.hzero;
+    TS zl = 0, zr = 0;  // boundary values (weights of hl / hr) of row lane % RPW, part (lane / RPW) % 2
+    if (bnd) {
+        const int rl = lane % RPW, part = (lane / RPW) & 1;
+        auto row = row_of(0);
+        int g = grp[0];
 #pragma unroll
-    for (int r = 0; r < RPW; ++r) {
-        if (!ok[r]) continue;  // warp-uniform
-        const auto row = row_of(r);
-        const int g = grp[r];
-        TS zlr = 0, zli = 0, zrr = 0, zri = 0;   // boundary values of the row (weights of hl / hr)
-        const bool bnd = a.hvec != nullptr;
-        if (bnd) {
-            // folded dot products with e0 / eN (forward: D0, DN rows; adjoint: D2 boundary columns)
-            TS p0r = 0, p0i = 0, pNr = 0, pNi = 0;
-#pragma unroll
-            for (int t = 0; t < NSS; ++t) {
-                const int k = lane + 32 * t;
-                if (k < ms) {
-                    const TS e0s = (TS)a.e0f[k], eNs = (TS)a.eNf[k];
-                    p0r += e0s * xsr[r][t]; p0i += e0s * xsi[r][t];
-                    pNr += eNs * xsr[r][t]; pNi += eNs * xsi[r][t];
-                }
-                if (k < ma) {
-                    const TS e0a = (TS)a.e0f[ld + k], eNa = (TS)a.eNf[ld + k];
-                    p0r += e0a * xdr[r][t]; p0i += e0a * xdi[r][t];
-                    pNr += eNa * xdr[r][t]; pNi += eNa * xdi[r][t];
-                }
+        for (int r = 1; r < RPW; ++r)
+            if (rl == r) {
+                row = row_of(r);
+                g = grp[r];
             }
-            p0r = wsum(p0r); p0i = wsum(p0i); pNr = wsum(pNr); pNi = wsum(pNi);
-            const CS wl = row.get(0), wr = row.get(P - 1);
-            const double* sc = a.hscal + (size_t)g * 4;
-            if (a.periodic) {
-                // periodic, one element (Periodic3D_MPI.cpp:322-333, 661-662): forward
-                // zeta = (DN - D0).phi / b; adjoint mu = (w0 + wN - c0.s - cN.s) / b,
-                // the same b = (D0 - DN).(ul + ur)
-                const TS bb = (TS)((sc[0] + sc[1]) - (sc[2] + sc[3]));
-                if (!ADJ) {
-                    zlr = (pNr - p0r) / bb; zli = (pNi - p0i) / bb;
-                } else {
-                    zlr = ((wl.x - p0r) + (wr.x - pNr)) / bb; zli = ((wl.y - p0i) + (wr.y - pNi)) / bb;
-                }
-                zrr = zlr; zri = zli;
-            } else if (!ADJ) {
-                // Robin ends, one element (NonPeriodic3D_MPI.cpp:334-336, 357-367, 528-529)
-                const TS b0 = (TS)(-a.al * sc[0] + a.bl), c0 = (TS)(-a.al * sc[1]);
-                const TS lb = (TS)(a.ar * sc[2]);
-                const TS bR = (TS)(a.ar * sc[3] + a.br) - (c0 / b0) * lb;
-                const TS rhr = wl.x + (TS)a.al * p0r, rhi = wl.y + (TS)a.al * p0i;
-                const TS rRr = wr.x - (TS)a.ar * pNr - (rhr / b0) * lb;
-                const TS rRi = wr.y - (TS)a.ar * pNi - (rhi / b0) * lb;
-                zrr = rRr / bR; zri = rRi / bR;
-                zlr = (rhr - c0 * zrr) / b0; zli = (rhi - c0 * zri) / b0;
-            } else {
-                const TS m00 = (TS)sc[0], m01 = (TS)sc[1], m10 = (TS)sc[2], m11 = (TS)sc[3];
-                const TS det = m00 * m11 - m01 * m10;
-                const TS q0r = wl.x - p0r, q0i = wl.y - p0i, qNr = wr.x - pNr, qNi = wr.y - pNi;
-                zlr = (m11 * q0r - m01 * qNr) / det; zli = (m11 * q0i - m01 * qNi) / det;
-                zrr = (m00 * qNr - m10 * q0r) / det; zri = (m00 * qNi - m10 * q0i) / det;
+        const CS w0 = row.get(0), wN = row.get(P - 1);
+        const double* scp = a.hscal + (size_t)g * 4;
+        const double sc[4] = {scp[0], scp[1], scp[2], scp[3]};
+        // folded dot products with e0 / eN (forward: D0, DN rows; adjoint: D2 boundary columns)
+        TS dots[4 * RPW];
+#pragma unroll
+        for (int i = 0; i < 4 * RPW; ++i) dots[i] = (TS)0;
+#pragma unroll
+        for (int t = 0; t < NSS; ++t) {
+            const int k = lane + 32 * t;
+            const TS e0s = k < ms ? (TS)a.e0f[k] : (TS)0, eNs = k < ms ? (TS)a.eNf[k] : (TS)0;
+            const TS e0a = k < ma ? (TS)a.e0f[ld + k] : (TS)0, eNa = k < ma ? (TS)a.eNf[ld + k] : (TS)0;
+#pragma unroll
+            for (int r = 0; r < RPW; ++r) {
+                // (folds past ms / ma are zero, or not to be read)
+                const TS sr = k < ms ? xsr[r][t] : (TS)0, si = k < ms ? xsi[r][t] : (TS)0;
+                const TS dr = k < ma ? xdr[r][t] : (TS)0, di = k < ma ? xdi[r][t] : (TS)0;
+                dots[4 * r] += e0s * sr;
+                dots[4 * r + 1] += e0s * si;
+                dots[4 * r + 2] += eNs * sr;
+                dots[4 * r + 3] += eNs * si;
+                dots[4 * r] += e0a * dr;
+                dots[4 * r + 1] += e0a * di;
+                dots[4 * r + 2] += eNa * dr;
+                dots[4 * r + 3] += eNa * di;
             }
         }
-        // the interior correction zl hl + zr hr (skipped when hl = hr = 0: the
-        // transposed system of Dirichlet ends)
-        const bool hadd = bnd && !a.hzero;
-        const double* hl = hadd ? a.hvec + (size_t)g * 2 * P : nullptr;
+        const TS sum = warp_sums<TS, 4 * RPW>(dots, lane);
+        auto lane_of = [](int i) { return (int)(__brev((unsigned)i) >> (32 - LOGV)); };
+        const TS p0 = __shfl_sync(0xffffffffu, sum, lane_of(4 * rl + part));
+        const TS pN = __shfl_sync(0xffffffffu, sum, lane_of(4 * rl + 2 + part));
+        const TS wl = part ? w0.y : w0.x, wr = part ? wN.y : wN.x;
+        if (a.periodic) {
+            // periodic, one element (Periodic3D_MPI.cpp:322-333, 661-662): forward
+            // zeta = (DN - D0).phi / b; adjoint mu = (w0 + wN - c0.s - cN.s) / b,
+            // the same b = (D0 - DN).(ul + ur)
+            const TS bb = (TS)((sc[0] + sc[1]) - (sc[2] + sc[3]));
+            zl = ADJ ? ((wl - p0) + (wr - pN)) / bb : (pN - p0) / bb;
+            zr = zl;
+        } else if (!ADJ) {
+            // Robin ends, one element (NonPeriodic3D_MPI.cpp:334-336, 357-367, 528-529)
+            const TS b0 = (TS)(-a.al * sc[0] + a.bl), c0 = (TS)(-a.al * sc[1]);
+            const TS lb = (TS)(a.ar * sc[2]);
+            const TS bR = (TS)(a.ar * sc[3] + a.br) - (c0 / b0) * lb;
+            const TS rh = wl + (TS)a.al * p0;
+            const TS rR = wr - (TS)a.ar * pN - (rh / b0) * lb;
+            zr = rR / bR;
+            zl = (rh - c0 * zr) / b0;
+        } else {
+            const TS m00 = (TS)sc[0], m01 = (TS)sc[1], m10 = (TS)sc[2], m11 = (TS)sc[3];
+            const TS det = m00 * m11 - m01 * m10;
+            const TS q0 = wl - p0, qN = wr - pN;
+            zl = (m11 * q0 - m01 * qN) / det;
+            zr = (m00 * qN - m10 * q0) / det;
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < RPW; ++r) {
+        TS zlr = 0, zli = 0, zrr = 0, zri = 0;
+        if (bnd) {
+            zlr = __shfl_sync(0xffffffffu, zl, r);
+            zli = __shfl_sync(0xffffffffu, zl, RPW + r);
+            zrr = __shfl_sync(0xffffffffu, zr, r);
+            zri = __shfl_sync(0xffffffffu, zr, RPW + r);
+        }
+        if (!ok[r]) continue;  // warp-uniform
+        const auto row = row_of(r);
+        const double* hl = hadd ? a.hvec + (size_t)grp[r] * 2 * P : nullptr;
         const double* hr = hadd ? hl + P : nullptr;
 #pragma unroll
         for (int t = 0; t < NSS; ++t) {
@@ -262,6 +306,18 @@ __device__ __forceinline__ void fdm_store_rows(const FdmArgs& a, cplx_t<TS>* spe
         lane);
 }
 
+// Rows and shift groups of pack pk (rows past the end: the first row's).
+template <int RPW>
+__device__ __forceinline__ void pack_ids(const FdmArgs& a, long long pk, int (&rowid)[RPW], int (&grp)[RPW])
+{
+#pragma unroll
+    for (int r = 0; r < RPW; ++r) {
+        const long long rr = pk * RPW + r;
+        rowid[r] = a.rows[rr < a.nrows ? rr : 0];
+        grp[r] = a.row_grp[rr < a.nrows ? rr : 0];
+    }
+}
+
 template <typename TS, typename TF, int NSS, int RPW, bool REFINE, bool ADJ>
 __global__ void __launch_bounds__(FDM_WARPS * 32, 2) fdm_fast_kernel(FdmArgs a)
 {
@@ -286,8 +342,6 @@ __global__ void __launch_bounds__(FDM_WARPS * 32, 2) fdm_fast_kernel(FdmArgs a)
         if (REFINE)
             for (int e = threadIdx.x; e < 2 * ld * ld; e += blockDim.x) Ms[e] = a.d2f[e];
     }
-    pdl_enter();  // the constants above are plan data; the spectrum comes from the previous pass
-    __syncthreads();
 
     CS* spec = static_cast<CS*>(a.spec);
     const TS r2 = (TS)0.70710678118654752440;  // fold weight, in the storage precision
@@ -295,17 +349,30 @@ __global__ void __launch_bounds__(FDM_WARPS * 32, 2) fdm_fast_kernel(FdmArgs a)
     const long long npacks = (nrows + RPW - 1) / RPW;
     const long long gw0 = (long long)blockIdx.x * FDM_WARPS + warp;
     const long long nw = (long long)gridDim.x * FDM_WARPS;
-
-    for (long long pk = gw0; pk < npacks; pk += nw) {
-        int rowid[RPW], grp[RPW];
-        bool ok[RPW];
+    // rows, shift groups and reciprocal shifts of a pack; all of it and the
+    // constants above are plan data, the spectrum comes from the previous pass
+    int rowid[RPW], grp[RPW];
+    TF rs[RPW][NSS], ra[RPW][NSS];
+    auto pack_data = [&](long long pk) {
+        pack_ids<RPW>(a, pk, rowid, grp);
 #pragma unroll
         for (int r = 0; r < RPW; ++r) {
-            const long long rr = pk * RPW + r;
-            ok[r] = rr < nrows;
-            rowid[r] = ok[r] ? a.rows[rr] : a.rows[0];
-            grp[r] = ok[r] ? a.row_grp[rr] : a.row_grp[0];
+            const TF* rc = static_cast<const TF*>(a.recip) + (size_t)grp[r] * 2 * ld;
+#pragma unroll
+            for (int t = 0; t < NSS; ++t) {
+                rs[r][t] = rc[lane + 32 * t];
+                ra[r][t] = rc[ld + lane + 32 * t];
+            }
         }
+    };
+    pack_data(gw0);
+    pdl_enter();
+    __syncthreads();
+
+    for (long long pk = gw0; pk < npacks; pk += nw) {
+        bool ok[RPW];
+#pragma unroll
+        for (int r = 0; r < RPW; ++r) ok[r] = pk * RPW + r < nrows;
         // ---- load the interior of each row and fold it ----
         TS fsr[RPW][NSS], fsi[RPW][NSS], fdr[RPW][NSS], fdi[RPW][NSS];
         {
@@ -333,17 +400,6 @@ __global__ void __launch_bounds__(FDM_WARPS * 32, 2) fdm_fast_kernel(FdmArgs a)
                     }
                     fsr[r][t] = a0; fsi[r][t] = a1; fdr[r][t] = b0; fdi[r][t] = b1;
                 }
-        }
-        // ---- reciprocal shifts of each row's group ----
-        TF rs[RPW][NSS], ra[RPW][NSS];
-#pragma unroll
-        for (int r = 0; r < RPW; ++r) {
-            const TF* rc = static_cast<const TF*>(a.recip) + (size_t)grp[r] * 2 * ld;
-#pragma unroll
-            for (int t = 0; t < NSS; ++t) {
-                rs[r][t] = rc[lane + 32 * t];
-                ra[r][t] = rc[ld + lane + 32 * t];
-            }
         }
         // ---- solve (+ FP64-residual refinement) in folded coordinates ----
         TF sr[RPW][NSS], si[RPW][NSS], dr[RPW][NSS], di[RPW][NSS];
@@ -430,6 +486,7 @@ __global__ void __launch_bounds__(FDM_WARPS * 32, 2) fdm_fast_kernel(FdmArgs a)
             }
         }
         fdm_store_rows<TS, NSS, RPW, ADJ>(a, spec, rowid, grp, ok, xsr, xsi, xdr, xdi, lane);
+        if (pk + nw < npacks) pack_data(pk + nw);
     }
 }
 
@@ -515,18 +572,41 @@ struct MmaShape {
     static constexpr size_t smem = (mats + (size_t)WARPS * 2 * RPW * RSD) * sizeof(double);
 };
 
-// Asynchronous copy of the interiors of pack pk's rows into stg (row r at
+// Asynchronous copy of the interiors of a pack's rows into stg (row r at
 // stg + r RSD, complex i at 2 i).
 template <int RPW, int RSD>
-__device__ __forceinline__ void mma_issue_pack(const FdmArgs& a, long long pk, double* stg, int lane)
+__device__ __forceinline__ void mma_issue_rows(const FdmArgs& a, const int (&rowid)[RPW], double* stg, int lane)
 {
     const cplx_t<double>* spec = static_cast<const cplx_t<double>*>(a.spec);
 #pragma unroll
     for (int r = 0; r < RPW; ++r) {
-        const long long rr = pk * RPW + r;
-        const int rowid = rr < a.nrows ? a.rows[rr] : a.rows[0];
-        const cplx_t<double>* row = spec + (long long)rowid * a.P + 1;
+        const cplx_t<double>* row = spec + (long long)rowid[r] * a.P + 1;
         for (int i = lane; i < a.n; i += 32) cp_async_bytes16(stg + r * RSD + 2 * i, row + i, true);
+    }
+}
+
+template <int RPW, int RSD>
+__device__ __forceinline__ void mma_issue_pack(const FdmArgs& a, long long pk, double* stg, int lane)
+{
+    int rowid[RPW], grp[RPW];
+    pack_ids<RPW>(a, pk, rowid, grp);
+    mma_issue_rows<RPW, RSD>(a, rowid, stg, lane);
+}
+
+// Reciprocal shifts 1 / (lambda_j - sigma) of this lane's accumulators in
+// mma_fold_solve: row 4 t + lane % 4 of shift group gq[t], fold index 8 mt + lane / 4.
+template <int NT, int MT, int LD>
+__device__ __forceinline__ void mma_recip(const double* recip, const int (&gq)[NT], double (&rs)[NT][MT],
+                                          double (&ra)[NT][MT], int lane)
+{
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+        const double* rc = recip + (size_t)gq[t] * 2 * LD + (lane >> 2);
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+            rs[t][mt] = rc[mt * 8];
+            ra[t][mt] = rc[LD + mt * 8];
+        }
     }
 }
 
@@ -534,10 +614,10 @@ __device__ __forceinline__ void mma_issue_pack(const FdmArgs& a, long long pk, d
 // stg + r RSD, complex i at 2 i), both transforms on the FP64 tensor cores
 // (mma.sync m8n8k4).  On return stg holds the folded solution: row r's
 // symmetric block at stg + r RSD + 2 i, its antisymmetric block at + 2 (LD + i).
-// gq[t]: shift group of row 4 t + (lane % 4).
+// rs, ra: mma_recip of the rows' shift groups.
 template <int NT, int MT, int KS, int RSD, int LD>
-__device__ __forceinline__ void mma_fold_solve(const double* A, const double* recip, double* stg, const int (&gq)[NT],
-                                               int n, int m, int ms, int lane)
+__device__ __forceinline__ void mma_fold_solve(const double* A, const double (&rs)[NT][MT], const double (&ra)[NT][MT],
+                                               double* stg, int n, int m, int ms, int lane)
 {
     const int g = lane >> 2, q = lane & 3;
     const double r2 = 0.70710678118654752440;
@@ -585,11 +665,10 @@ __device__ __forceinline__ void mma_fold_solve(const double* A, const double* re
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
         const int r = 4 * t + q;
-        const double* rc = recip + (size_t)gq[t] * 2 * LD;
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt) {
             const int i = mt * 8 + g;
-            const double s = rc[i], u = rc[LD + i];
+            const double s = rs[t][mt], u = ra[t][mt];
             *reinterpret_cast<double2*>(stg + r * RSD + 2 * i) = make_double2(cs[t][mt][0] * s, cs[t][mt][1] * s);
             *reinterpret_cast<double2*>(stg + r * RSD + 2 * (LD + i)) =
                 make_double2(ca[t][mt][0] * u, ca[t][mt][1] * u);
@@ -648,41 +727,44 @@ __global__ void __launch_bounds__(WARPS * 32, (NSS == 1 ? 2 : 1)) fdm_mma_kernel
         double2* dst = reinterpret_cast<double2*>(A);
         for (int e = threadIdx.x; e < (int)(S::mats / 2); e += blockDim.x) dst[e] = src[e];
     }
+    // plan data of the first pack, before the previous pass's results are waited for
+    const int n = a.n, m = a.m, ms = a.ms, nrows = a.nrows;
+    const long long npacks = (nrows + RPW - 1) / RPW;
+    const long long pstride = (long long)gridDim.x * WARPS;
+    long long pk = (long long)blockIdx.x * WARPS + warp;
+    int rowid[RPW], grp[RPW];
+    double rs[NT][MT], ra[NT][MT];
+    auto recips = [&]() {
+        int gq[NT];
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+            gq[t] = q & 2 ? (q & 1 ? grp[4 * t + 3] : grp[4 * t + 2]) : (q & 1 ? grp[4 * t + 1] : grp[4 * t]);
+        mma_recip<NT, MT, LD>(static_cast<const double*>(a.recip), gq, rs, ra, lane);
+    };
+    pack_ids<RPW>(a, pk, rowid, grp);
+    recips();
     pdl_enter();
     __syncthreads();
 
     cplx_t<double>* spec = static_cast<cplx_t<double>*>(a.spec);
-    const int n = a.n, m = a.m, ms = a.ms, nrows = a.nrows;
-    const long long npacks = (nrows + RPW - 1) / RPW;
-
-    const long long pstride = (long long)gridDim.x * WARPS;
-    long long pk = (long long)blockIdx.x * WARPS + warp;
     int cur = 0;
-    if (pk < npacks) mma_issue_pack<RPW, RSD>(a, pk, stg_base, lane);
+    if (pk < npacks) mma_issue_rows<RPW, RSD>(a, rowid, stg_base, lane);
     cp_async_commit();
     for (; pk < npacks; pk += pstride, cur ^= 1) {
         double* stg = stg_base + (size_t)cur * RPW * RSD;
-        if (pk + pstride < npacks) mma_issue_pack<RPW, RSD>(a, pk + pstride, stg_base + (size_t)(cur ^ 1) * RPW * RSD, lane);
+        int nrow[RPW], ngrp[RPW];
+        if (pk + pstride < npacks) {
+            pack_ids<RPW>(a, pk + pstride, nrow, ngrp);
+            mma_issue_rows<RPW, RSD>(a, nrow, stg_base + (size_t)(cur ^ 1) * RPW * RSD, lane);
+        }
         cp_async_commit();
-        int rowid[RPW], grp[RPW];
         bool ok[RPW];
 #pragma unroll
-        for (int r = 0; r < RPW; ++r) {
-            const long long rr = pk * RPW + r;
-            ok[r] = rr < nrows;
-            rowid[r] = ok[r] ? a.rows[rr] : a.rows[0];
-            grp[r] = ok[r] ? a.row_grp[rr] : a.row_grp[0];
-        }
+        for (int r = 0; r < RPW; ++r) ok[r] = pk * RPW + r < nrows;
         // ---- the staged interiors of this pack's rows ----
         cp_async_wait_prev();
         __syncwarp();
-        int gq[NT];
-#pragma unroll
-        for (int t = 0; t < NT; ++t) {
-            const long long rr = pk * RPW + 4 * t + q;
-            gq[t] = a.row_grp[rr < nrows ? rr : 0];
-        }
-        mma_fold_solve<NT, MT, KS, RSD, LD>(A, static_cast<const double*>(a.recip), stg, gq, n, m, ms, lane);
+        mma_fold_solve<NT, MT, KS, RSD, LD>(A, rs, ra, stg, n, m, ms, lane);
         // ---- folded solution to the lane-per-fold-index layout, epilogue ----
         double xsr[RPW][NSS], xsi[RPW][NSS], xdr[RPW][NSS], xdi[RPW][NSS];
 #pragma unroll
@@ -696,6 +778,14 @@ __global__ void __launch_bounds__(WARPS * 32, (NSS == 1 ? 2 : 1)) fdm_mma_kernel
             }
         fdm_store_rows<double, NSS, RPW, ADJ>(a, spec, rowid, grp, ok, xsr, xsi, xdr, xdi, lane);
         __syncwarp();  // stg is refilled by the copy issued in the next iteration
+        if (pk + pstride < npacks) {
+#pragma unroll
+            for (int r = 0; r < RPW; ++r) {
+                rowid[r] = nrow[r];
+                grp[r] = ngrp[r];
+            }
+            recips();
+        }
     }
     cp_async_wait_all();
 }
@@ -748,8 +838,6 @@ __global__ void __launch_bounds__(WARPS * 32, (NSS == 1 ? 2 : 1)) fdm_mma16_kern
         double2* dst = reinterpret_cast<double2*>(A);
         for (int e = threadIdx.x; e < (int)(S::mats / 2); e += blockDim.x) dst[e] = src[e];
     }
-    pdl_enter();
-    __syncthreads();
 
     cplx_t<double>* spec = static_cast<cplx_t<double>*>(a.spec);
     const int n = a.n, m = a.m, ms = a.ms, nrows = a.nrows;
@@ -763,34 +851,38 @@ __global__ void __launch_bounds__(WARPS * 32, (NSS == 1 ? 2 : 1)) fdm_mma16_kern
     const long long pstride = (long long)gridDim.x * WARPS;
     long long pk = (long long)blockIdx.x * WARPS + warp;
     int cur = 0;
-    if (pk < npacks) mma_issue_pack<RPW, RSD>(a, pk, stg_base, lane);
+    // plan data of the first pack (rows, reciprocal shifts of this lane's
+    // accumulator rows), before the previous pass's results are waited for
+    int rowid[RPW], grp[RPW];
+    double rs[MT][2], ra[MT][2];
+    auto recips = [&]() {
+        const int gq = q & 2 ? (q & 1 ? grp[3] : grp[2]) : (q & 1 ? grp[1] : grp[0]);
+        const double* rc = rcp + (size_t)gq * 2 * LD;
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+            rs[mt][0] = rc[mt * 16 + g];
+            rs[mt][1] = rc[mt * 16 + g + 8];
+            ra[mt][0] = rc[LD + mt * 16 + g];
+            ra[mt][1] = rc[LD + mt * 16 + g + 8];
+        }
+    };
+    pack_ids<RPW>(a, pk, rowid, grp);
+    recips();
+    pdl_enter();
+    __syncthreads();
+    if (pk < npacks) mma_issue_rows<RPW, RSD>(a, rowid, stg_base, lane);
     cp_async_commit();
     for (; pk < npacks; pk += pstride, cur ^= 1) {
         double* stg = stg_base + (size_t)cur * RPW * RSD;
-        if (pk + pstride < npacks) mma_issue_pack<RPW, RSD>(a, pk + pstride, stg_base + (size_t)(cur ^ 1) * RPW * RSD, lane);
+        int nrow[RPW], ngrp[RPW];
+        if (pk + pstride < npacks) {
+            pack_ids<RPW>(a, pk + pstride, nrow, ngrp);
+            mma_issue_rows<RPW, RSD>(a, nrow, stg_base + (size_t)(cur ^ 1) * RPW * RSD, lane);
+        }
         cp_async_commit();
-        int rowid[RPW], grp[RPW];
         bool ok[RPW];
 #pragma unroll
-        for (int r = 0; r < RPW; ++r) {
-            const long long rr = pk * RPW + r;
-            ok[r] = rr < nrows;
-            rowid[r] = ok[r] ? a.rows[rr] : a.rows[0];
-            grp[r] = ok[r] ? a.row_grp[rr] : a.row_grp[0];
-        }
-        // reciprocal shifts of this lane's accumulator rows (row q), loaded early
-        double rs[MT][2], ra[MT][2];
-        {
-            const int gq = a.row_grp[(pk * RPW + q) < nrows ? pk * RPW + q : 0];
-            const double* rc = rcp + (size_t)gq * 2 * LD;
-#pragma unroll
-            for (int mt = 0; mt < MT; ++mt) {
-                rs[mt][0] = rc[mt * 16 + g];
-                rs[mt][1] = rc[mt * 16 + g + 8];
-                ra[mt][0] = rc[LD + mt * 16 + g];
-                ra[mt][1] = rc[LD + mt * 16 + g + 8];
-            }
-        }
+        for (int r = 0; r < RPW; ++r) ok[r] = pk * RPW + r < nrows;
         cp_async_wait_prev();
         __syncwarp();
         // ---- first transform; B fragments folded on the fly ----
@@ -883,6 +975,14 @@ __global__ void __launch_bounds__(WARPS * 32, (NSS == 1 ? 2 : 1)) fdm_mma16_kern
             }
         fdm_store_rows<double, NSS, RPW, ADJ>(a, spec, rowid, grp, ok, xsr, xsi, xdr, xdi, lane);
         __syncwarp();  // stg is refilled by the copy issued in the next iteration
+        if (pk + pstride < npacks) {
+#pragma unroll
+            for (int r = 0; r < RPW; ++r) {
+                rowid[r] = nrow[r];
+                grp[r] = ngrp[r];
+            }
+            recips();
+        }
     }
     cp_async_wait_all();
 }
@@ -1026,7 +1126,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(SLAB_WARPS * 32, 1) 
         }
         __syncwarp();
         int gq[1] = {sa.grp_of_row[(long long)kx * L + kyb + q]};
-        mma_fold_solve<1, MT, KS, RSD, LD>(A, static_cast<const double*>(a.recip), stg, gq, n, m, ms, lane);
+        double rs[1][MT], ra[1][MT];
+        mma_recip<1, MT, LD>(static_cast<const double*>(a.recip), gq, rs, ra, lane);
+        mma_fold_solve<1, MT, KS, RSD, LD>(A, rs, ra, stg, n, m, ms, lane);
         double xsr[RPW][1], xsi[RPW][1], xdr[RPW][1], xdi[RPW][1];
         int grp[RPW];
         bool ok[RPW];
