@@ -6,6 +6,7 @@
 //     u = phi + zl ul + zr ur (:466-470), fused, one warp per complex row (the LU
 //     method; fast-diagonalisation plans with several elements: helm_multi.cu).
 #include <algorithm>
+#include <type_traits>
 
 #include "helm_device.cuh"
 #include "helm_kernels.cuh"
@@ -764,7 +765,7 @@ __global__ void __launch_bounds__(TRI_WARPS * 32, (M <= 8 ? 4 : (sizeof(T) == 8 
             if (k == Nz - 1) b += a.d_last;
             return (T)b;
         };
-        const int k0 = li * M;
+        const int k0 = li * M, last = Nz - 1 - k0;  // the last row's place in the chunk
         // ---- 1. eliminate the lane's interior rows ----
         TriEq<T> e0, e1;
         C y[M > 2 ? M - 2 : 1];
@@ -775,18 +776,43 @@ __global__ void __launch_bounds__(TRI_WARPS * 32, (M <= 8 ? 4 : (sizeof(T) == 8 
         } else {
             constexpr int NI = M - 2;
             T cp[NI];
+            // Rows k0 + 1 .. k0 + M - 2 (never the first): cz dg cz, but for the last
+            // row and its neighbour, the identity rows past it, and row 1 of the
+            // transposed matrix.  A warp whose lanes all lie inside takes the
+            // constants as they stand: 1024 x 1024 modes of 256 points, FP64, 1029 ->
+            // 880 us (transposed 958), 512 x 512 of 128 152 -> 124 us; chunks that
+            // the row ends in, 256 x 128 of 100, FP32 21.4 -> 19.3 us.
+            const T dgT = (T)dg, dlast = (T)(dg + a.d_last);
+            const T sub1 = (a.transpose && k0 == 0) ? (T)a.s_first : cz;
+            const T sublast = a.transpose ? cz : (T)a.s_last, suplast = a.transpose ? (T)a.s_last : cz;
+            auto eliminate = [&](auto inside) {
+                constexpr bool IN = decltype(inside)::value;
 #pragma unroll
-            for (int j = 0; j < NI; ++j) {
-                const int k = k0 + j + 1;
-                const T al = (j > 0) ? sub(k) : (T)0;
-                const T den = (j > 0) ? dia(k) - al * cp[j - 1] : dia(k);
-                const T m = (T)1 / den;
-                cp[j] = (j < NI - 1) ? sup(k) * m : (T)0;
-                const C yp = (j > 0) ? y[j - 1] : mk((T)0, (T)0);
-                y[j] = mk((dv[j + 1].x - al * yp.x) * m, (dv[j + 1].y - al * yp.y) * m);
-                v[j] = (((j == 0) ? sub(k) : (T)0) - ((j > 0) ? al * v[j - 1] : (T)0)) * m;
-                w[j] = (((j == NI - 1) ? sup(k) : (T)0) - ((j > 0) ? al * w[j - 1] : (T)0)) * m;
-            }
+                for (int j = 0; j < NI; ++j) {
+                    const int jj = j + 1;
+                    T al = jj == 1 ? sub1 : cz, b = dgT, c = cz;
+                    if (!IN) {
+                        if (jj == last && !a.transpose) al = sublast;
+                        al = jj > last ? (T)0 : al;
+                        b = jj < last ? dgT : jj == last ? dlast : (T)1;
+                        c = jj + 1 < last ? cz : jj + 1 == last ? suplast : (T)0;
+                    }
+                    const T m = (T)1 / ((j > 0) ? b - al * cp[j > 0 ? j - 1 : 0] : b);
+                    cp[j] = (j < NI - 1) ? c * m : (T)0;
+                    if (j == 0) {
+                        y[0] = mk(dv[1].x * m, dv[1].y * m);
+                        v[0] = al * m;
+                        w[0] = NI == 1 ? c * m : (T)0;
+                    } else {
+                        const C yp = y[j > 0 ? j - 1 : 0];
+                        y[j] = mk((dv[jj].x - al * yp.x) * m, (dv[jj].y - al * yp.y) * m);
+                        v[j] = -(al * v[j > 0 ? j - 1 : 0]) * m;
+                        w[j] = (j == NI - 1) ? c * m : (T)0;
+                    }
+                }
+            };
+            if (__all_sync(0xffffffffu, last >= M - (a.transpose ? 0 : 1))) eliminate(std::true_type{});
+            else eliminate(std::false_type{});
 #pragma unroll
             for (int j = NI - 2; j >= 0; --j) {
                 y[j] = mk(y[j].x - cp[j] * y[j + 1].x, y[j].y - cp[j] * y[j + 1].y);
