@@ -315,9 +315,12 @@ template <typename TS, int NT>
 int run_multi(MultiArgs a, cudaStream_t s)
 {
     auto k = a.adjoint ? multi_rows_kernel<TS, NT, true> : multi_rows_kernel<TS, NT, false>;
-    // Rows per CTA: enough vectors for eight warps (32: four per warp) when the
-    // elements are few, while every SM still gets two CTAs.
-    int R = 32 / a.Ns;
+    // Rows per CTA: 64 vectors, two groups of four for each of eight warps, when the
+    // elements are few, while every SM still gets two CTAs.  With 32 vectors a
+    // CTA's fixed costs (plan data, barriers, the sweep) weighed twice as much: 14.6
+    // against 18.6 us (stage, between events) for 1056 rows of 25 x 10 points,
+    // 18.3 against 22.4 for 2112 of 6 x 20; 52 x 10 on 257 rows is the same 14.7.
+    int R = 64 / a.Ns;
     const int most = (a.nrows + 2 * 148 - 1) / (2 * 148);
     if (R > most) R = most;
     if (R < 1) R = 1;
@@ -328,8 +331,12 @@ int run_multi(MultiArgs a, cudaStream_t s)
     cudaError_t e = allow_smem(k, smem);
     if (e != cudaSuccess) return (int)e;
     const int tasks = (R * a.Ns + 3) / 4;
-    const int threads = tasks >= 5 ? 256 : tasks >= 3 ? 128 : 64;
-    return (int)launch_k(k, dim3((a.nrows + R - 1) / R), dim3(threads), smem, s, a);
+    const int ctas = (a.nrows + R - 1) / R;
+    // Beyond eight CTAs an SM in all, four warps each: more CTAs side by side hide
+    // one another's barriers (4160 of 2 x 30 x 6 points 43 us, eight warps 53; but
+    // 528 of 2 x 25 x 10 15.5 and 14.6).
+    const int threads = (tasks >= 5 && ctas <= 8 * 148) ? 256 : tasks >= 3 ? 128 : 64;
+    return (int)launch_k(k, dim3(ctas), dim3(threads), smem, s, a);
 }
 
 template <typename TS>
