@@ -269,17 +269,24 @@ static int setup_multi(Plan& p, const std::vector<double>& V, const std::vector<
     std::vector<int> gor((size_t)p.nrows, 0);
     for (int g = 0; g < G; ++g)
         for (int rr = p.grp_start[g]; rr < p.grp_start[g + 1]; ++rr) gor[p.grp_rows[rr]] = g;
-    int st;
-    auto up = [&](const std::vector<double>& h, double** d) { return p.upload((void**)d, h.data(), h.size() * sizeof(double)); };
-    if ((st = up(multi_fragments1(n, Vi.data()), &p.d_mm1))) return st;
-    if ((st = up(multi_fragments2(n, n + 2, vs.data()), &p.d_mm2))) return st;
-    if ((st = up(f, &p.d_itf))) return st;
-    if ((st = p.upload((void**)&p.d_grp_of_row, gor.data(), gor.size() * sizeof(int)))) return st;
-    if (!p.periodic) {
-        if ((st = up(multi_fragments1(n, vt.data()), &p.d_mm1_adj))) return st;
-        if ((st = up(multi_fragments2(n, n, vit.data()), &p.d_mm2_adj))) return st;
-        p.adj_ready = true;
+    // one allocation and copy for all of it
+    const std::vector<double> parts[5] = {multi_fragments1(n, Vi.data()), multi_fragments2(n, n + 2, vs.data()), f,
+                                          p.periodic ? std::vector<double>() : multi_fragments1(n, vt.data()),
+                                          p.periodic ? std::vector<double>() : multi_fragments2(n, n, vit.data())};
+    double** const dst[5] = {&p.d_mm1, &p.d_mm2, &p.d_itf, &p.d_mm1_adj, &p.d_mm2_adj};
+    std::vector<double> all;
+    size_t at[5];
+    for (int i = 0; i < 5; ++i) {
+        at[i] = all.size();
+        all.insert(all.end(), parts[i].begin(), parts[i].end());
+        all.resize((all.size() + 15) / 16 * 16, 0.0);
     }
+    double* base = nullptr;
+    int st;
+    if ((st = p.upload((void**)&base, all.data(), all.size() * sizeof(double)))) return st;
+    if ((st = p.upload((void**)&p.d_grp_of_row, gor.data(), gor.size() * sizeof(int)))) return st;
+    for (int i = 0; i < 5; ++i) *dst[i] = parts[i].empty() ? nullptr : base + at[i];
+    if (!p.periodic) p.adj_ready = true;
     p.multi = true;
     return HELM_OK;
 }
