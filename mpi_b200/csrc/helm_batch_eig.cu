@@ -196,24 +196,55 @@ __device__ __forceinline__ double be_mu(const BeClass& c, int j, bool& live)
     return live ? c.mu[j < ld ? j : c.ms + (j - ld)] : 0.0;
 }
 
-// Kind 2: column pairs [16 idx, 16 idx + CT) of problem pr, along x.
+// The passes of a length-L transform after its first, whose outputs v holds: back
+// with the last pass's outputs (item (t, r) at row slab_out_row<RL, L / RL>).
+template <int L, int DIR, int TPC, class RS>
+__device__ __forceinline__ void be_later_passes(double2* z, int HS, const double2* tw, int tc, int cl, bool on,
+                                                double2 (&v)[RS::r0])
+{
+    constexpr int R0 = RS::r0, R1 = RS::r1, R2 = RS::r2;
+    if constexpr (RS::n >= 2) {
+        if (on) slab_to_smem<L, R0, 1, TPC, R0>(z, HS, tc, cl, v);
+        __syncthreads();
+        if (on) slab_from_smem<L, R1, R0, DIR, TPC, R0>(z, HS, tw, tc, cl, v);
+    }
+    if constexpr (RS::n >= 3) {
+        __syncthreads();
+        if (on) slab_to_smem<L, R1, R0, TPC, R0>(z, HS, tc, cl, v);
+        __syncthreads();
+        if (on) slab_from_smem<L, R2, R0 * R1, DIR, TPC, R0>(z, HS, tw, tc, cl, v);
+    }
+}
+
+// Kind 2: column pairs [16 idx, 16 idx + CT) of problem pr, along x.  The columns
+// come from and go back to the scratch straight from the registers of the first and
+// last pass; the last forward pass writes the rows its thread read, so only the
+// split and the passes between wait for one another.
 template <int L>
 __device__ void be_columns(const BeArgs& a, const BeProblem& pr, const BeClass& c, int idx, double* sm)
 {
     constexpr int LOG2 = L == 8 ? 3 : L == 16 ? 4 : L == 32 ? 5 : L == 64 ? 6 : L == 128 ? 7 : L == 256 ? 8 : 9;
-    const int ld2 = 2 * c.ld, CT = be_cols(L, c.ld), col0 = idx * 2 * CT, HS = CT + 1;
+    const int CT = be_cols(L, c.ld), col0 = idx * 2 * CT, HS = CT + 1;
     double2* z = reinterpret_cast<double2*>(sm);  // [L][HS]
     double* Cb = a.C + pr.coff;
-    for (int e = threadIdx.x; e < L * CT; e += BE_THREADS) {
-        const int x = e / CT, cc = e - x * CT;
-        cp_async_bytes16(&z[x * HS + cc], Cb + (long long)x * ld2 + col0 + 2 * cc, true);
-    }
-    cp_async_commit();
-    cp_async_wait_all();
-    __syncthreads();
     const double2* tw = a.tw[LOG2];
     using RS = typename std::conditional<L == 512, Radix512Wide, Radix<L>>::type;
-    slab_fft<L, -1, BE_THREADS, 0, 1, RS>(z, HS, CT, tw);
+    constexpr int R0 = RS::r0, RL = RS::n == 1 ? R0 : RS::n == 2 ? RS::r1 : RS::r2;
+    constexpr int TPC = L / R0, CPR = BE_THREADS / TPC;
+    const int tc = threadIdx.x / CPR, cl = threadIdx.x - tc * CPR;
+    const bool on = cl < CT;
+    double2* col = reinterpret_cast<double2*>(Cb + col0) + cl;  // row x at + x ld
+    const int ld = c.ld;
+    {
+        double2 v[R0];
+        // (other CTAs wrote them: past L1)
+#pragma unroll
+        for (int r = 0; r < R0; ++r) v[r] = on ? __ldcg(col + (long long)(tc + r * TPC) * ld) : make_double2(0.0, 0.0);
+        dft_reg<R0, -1, double>(v);
+        be_later_passes<L, -1, TPC, RS>(z, HS, tw, tc, cl, on, v);
+        if (on) slab_to_smem<L, RL, L / RL, TPC, R0>(z, HS, tc, cl, v);
+    }
+    __syncthreads();
     // real-to-complex split of each column pair, scaling, and the assembly of
     // the full-length spectrum for the inverse (imaginary parts dropped at
     // kx = 0 and L / 2)
@@ -237,11 +268,18 @@ __device__ void be_columns(const BeArgs& a, const BeProblem& pr, const BeClass& 
         if (kx > 0 && kx < L / 2) z[km * HS + cc] = make_double2(X.x + Y.y, Y.x - X.y);
     }
     __syncthreads();
-    slab_fft<L, 1, BE_THREADS, 0, 1, RS>(z, HS, CT, tw);
-    for (int e = threadIdx.x; e < L * CT; e += BE_THREADS) {
-        const int x = e / CT, cc = e - x * CT;
-        __stcg(reinterpret_cast<double2*>(Cb + (long long)x * ld2 + col0 + 2 * cc), z[x * HS + cc]);
-    }
+    double2 v[R0];
+#pragma unroll
+    for (int r = 0; r < R0; ++r) v[r] = on ? z[(tc + r * TPC) * HS + cl] : make_double2(0.0, 0.0);
+    dft_reg<R0, 1, double>(v);
+    if constexpr (RS::n >= 2) __syncthreads();  // every row is read before the exchange overwrites it
+    be_later_passes<L, 1, TPC, RS>(z, HS, tw, tc, cl, on, v);
+    if (on)
+#pragma unroll
+        for (int t = 0; t < R0 / RL; ++t)
+#pragma unroll
+            for (int r = 0; r < RL; ++r)
+                __stcg(col + (long long)slab_out_row<RL, L / RL, TPC>(tc, t, r) * ld, v[t * RL + r]);
 }
 
 // Kind 3: coefficient rows x0 .. x0+R-1 -> second transform, unfold -> u rows.
