@@ -274,6 +274,18 @@ __device__ __forceinline__ cplx_t<T> deriv_mul_packed(int order, double w, int k
     return mk(m * Z.x, m * Z.y);
 }
 
+// Batch and column within it of column g < total; 64-bit division only where needed.
+__device__ __forceinline__ void split_column(long long g, int ccols, long long total, int& b, int& c)
+{
+    if (total <= 0x7fffffff) {
+        b = (int)((unsigned)g / (unsigned)ccols);
+        c = (int)((unsigned)g - (unsigned)b * (unsigned)ccols);
+    } else {
+        b = (int)(g / ccols);
+        c = (int)(g - (long long)b * ccols);
+    }
+}
+
 // Warps an SM has room for: 24 (at most 85 registers a thread), or 16 where 16
 // points of 8 bytes a thread, or an adjoint pass's operands, would spill at that.
 template <typename T, typename TIO, int L, int MODE, int THREADS, int SMALL>
@@ -287,8 +299,6 @@ constexpr int fft_min_ctas()
 template <typename T, typename TIO, int L, int DIR, int MODE, int THREADS, int SMALL>
 __global__ void __launch_bounds__(THREADS, (fft_min_ctas<T, TIO, L, MODE, THREADS, SMALL>())) fft_kernel(FftArgs a, long long total_cols)
 {
-    pdl_enter();
-    if (a.zero_out && blockIdx.x == 0 && threadIdx.x == 0) *a.zero_out = 0.0;
     using C = cplx_t<T>;
     using S = FftShape<T, L, THREADS, SMALL>;
     constexpr int R0 = S::R0, R1 = S::R1, R2 = S::R2, NP = S::NP, TPC = S::TPC, CT = S::CT;
@@ -301,13 +311,15 @@ __global__ void __launch_bounds__(THREADS, (fft_min_ctas<T, TIO, L, MODE, THREAD
     const long long g = (long long)blockIdx.x * CT + cl;
     const bool valid = g < total_cols;
     const int ccols = (MODE == FFT_C2C) ? a.ncols : (a.ncols + 1) >> 1;
-    const long long gg = valid ? g : 0;
-    const int b = (int)(gg / ccols);
-    const int c = (int)(gg - (long long)b * ccols);
+    int b, c;
+    split_column(valid ? g : 0, ccols, total_cols, b, c);
     const int c0 = 2 * c, c1 = 2 * c + 1;  // real columns of an R2C / C2R pair
     const bool has1 = c1 < a.ncols;
     const long long in_base = a.in_boff ? a.in_boff[b] : (long long)b * a.in_batch;
     const long long out_base = a.out_boff ? a.out_boff[b] : (long long)b * a.out_batch;
+    // (the columns' addresses are plan data: worked out before the previous pass is waited for)
+    pdl_enter();
+    if (a.zero_out && blockIdx.x == 0 && threadIdx.x == 0) *a.zero_out = 0.0;
 
     C v[R0];
     // ---------------------------------------------------------- pass 0 --
@@ -548,9 +560,8 @@ __device__ __forceinline__ void pipe_issue(const FftArgs& a, long long total_col
     const long long g = tile * CT + cl;
     const bool valid = g < total_cols;
     const int ccols = (MODE == FFT_C2C) ? a.ncols : (a.ncols + 1) >> 1;
-    const long long gg = valid ? g : 0;
-    const int b = (int)(gg / ccols);
-    const int c = (int)(gg - (long long)b * ccols);
+    int b, c;
+    split_column(valid ? g : 0, ccols, total_cols, b, c);
     const long long in_base = a.in_boff ? a.in_boff[b] : (long long)b * a.in_batch;
     if constexpr (MODE == FFT_C2C) {
         const C* in = static_cast<const C*>(a.in) + in_base;
@@ -620,9 +631,8 @@ __global__ void __launch_bounds__(THREADS) fft_pipe_kernel(FftArgs a, long long 
         C* sm = reinterpret_cast<C*>(buf);
         const long long g = tile * CT + cl;
         const bool valid = g < total_cols;
-        const long long gg = valid ? g : 0;
-        const int b = (int)(gg / ccols);
-        const int c = (int)(gg - (long long)b * ccols);
+        int b, c;
+        split_column(valid ? g : 0, ccols, total_cols, b, c);
         const int c0 = 2 * c, c1 = 2 * c + 1;
         const bool has1 = c1 < a.ncols;
         const long long out_base = a.out_boff ? a.out_boff[b] : (long long)b * a.out_batch;
