@@ -144,6 +144,17 @@ template <> struct RadixV<128, 1> { static constexpr int n = 3, r0 = 8, r1 = 4, 
 template <> struct RadixV<256, 1> { static constexpr int n = 3, r0 = 8, r1 = 8, r2 = 4; };
 template <int L> constexpr bool has_small_radix() { return L == 128 || L == 256; }
 
+// Where row `row` of the exchange after a first pass of radix R0 lies when the
+// columns of a row fill `bytes` < 128 bytes: threads one apart write rows R0
+// apart, all to the same banks, so the rows of every block of R0 change places by
+// the block's number.
+template <int R0>
+__device__ __forceinline__ int swizzle_row(int row, size_t bytes)
+{
+    const int mask = bytes >= 128 ? 0 : (int)(128 / bytes) - 1;
+    return mask < R0 ? row ^ ((row / R0) & mask) : row;
+}
+
 // The inverse of a length-L forward transform whose last pass has left its outputs
 // in registers (item (t, r) of radix RL at row tc + t TPC + r L / RL): the same
 // passes backwards, each radix-R butterfly before its conjugated twiddles.  No
@@ -151,7 +162,8 @@ template <int L> constexpr bool has_small_radix() { return L == 128 || L == 256;
 // order would need: one exchange fewer through shared memory.  sm: the exchange
 // buffer [L][hs], column cl; on return v[r] holds row tc + r TPC, unscaled.  All
 // threads of the CTA call it; the first write goes to the rows this thread read
-// last, so it needs no barrier before it.
+// last, so it needs no barrier before it.  SW: the exchange of the radix-R0 pass is
+// swizzled (swizzle_row), as it has to be in a forward transform of two passes then.
 template <int R, int NS, int TPC, int L, int R0, typename T>
 __device__ __forceinline__ void mirror_pass(const cplx_t<T>* tw, int tc, cplx_t<T> (&v)[R0])
 {
@@ -167,7 +179,7 @@ __device__ __forceinline__ void mirror_pass(const cplx_t<T>* tw, int tc, cplx_t<
     }
 }
 
-template <typename T, int L, int TPC, int R0, int R1, int R2, int NP>
+template <typename T, int L, int TPC, int R0, int R1, int R2, int NP, bool SW = false>
 __device__ __forceinline__ void fft_inverse_mirror(cplx_t<T>* sm, int hs, const cplx_t<T>* tw, int tc, int cl,
                                                    cplx_t<T> (&v)[R0])
 {
@@ -195,10 +207,13 @@ __device__ __forceinline__ void fft_inverse_mirror(cplx_t<T>* sm, int hs, const 
 #pragma unroll
         for (int t = 0; t < R0 / R1; ++t)
 #pragma unroll
-            for (int r = 0; r < R1; ++r) sm[(tc + t * TPC + r * (L / R1)) * hs + cl] = v[t * R1 + r];
+            for (int r = 0; r < R1; ++r) {
+                const int row = tc + t * TPC + r * (L / R1);
+                sm[(SW ? swizzle_row<R0>(row, hs * sizeof(cplx_t<T>)) : row) * hs + cl] = v[t * R1 + r];
+            }
         __syncthreads();
 #pragma unroll
-        for (int r = 0; r < R0; ++r) v[r] = sm[(tc * R0 + r) * hs + cl];
+        for (int r = 0; r < R0; ++r) v[r] = sm[(SW ? swizzle_row<R0>(tc * R0 + r, hs * sizeof(cplx_t<T>)) : tc * R0 + r) * hs + cl];
     }
     dft_reg<R0, 1, T>(v);
 }

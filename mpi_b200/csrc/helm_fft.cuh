@@ -47,7 +47,7 @@ __device__ __forceinline__ void dft_sub(cplx_t<T>* v)
 
 // One Stockham pass (radix R, NS = product of the earlier radices) reading
 // shared memory: every thread loads, twiddles and transforms its R0/R items.
-template <typename T, int L, int R, int NS, int DIR, int TPC, int CT, int R0>
+template <typename T, int L, int R, int NS, int DIR, int TPC, int CT, int R0, bool SW = false>
 __device__ __forceinline__ void pass_from_smem(const cplx_t<T>* sm, const cplx_t<T>* tw, int tc, int cl,
                                                cplx_t<T> (&v)[R0])
 {
@@ -58,7 +58,8 @@ __device__ __forceinline__ void pass_from_smem(const cplx_t<T>* sm, const cplx_t
         const int jm = j % NS;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            cplx_t<T> x = sm[(j + r * (L / R)) * CT + cl];
+            const int row = j + r * (L / R);
+            cplx_t<T> x = sm[(SW ? swizzle_row<R0>(row, CT * sizeof(cplx_t<T>)) : row) * CT + cl];
             if (NS > 1 && r > 0) {
                 const cplx_t<T> w = tw[r * jm * (L / (NS * R))];
                 x = (DIR < 0) ? cmul(x, w) : cmulc(x, w);
@@ -77,13 +78,16 @@ __device__ __forceinline__ int pass_out_row(int tc, int t, int r)
     return (j / NS) * NS * R + (j % NS) + r * NS;
 }
 
-template <typename T, int L, int R, int NS, int TPC, int CT, int R0>
+template <typename T, int L, int R, int NS, int TPC, int CT, int R0, bool SW = false>
 __device__ __forceinline__ void pass_to_smem(cplx_t<T>* sm, int tc, int cl, const cplx_t<T> (&v)[R0])
 {
 #pragma unroll
     for (int t = 0; t < R0 / R; ++t)
 #pragma unroll
-        for (int r = 0; r < R; ++r) sm[pass_out_row<R, NS, TPC>(tc, t, r) * CT + cl] = v[t * R + r];
+        for (int r = 0; r < R; ++r) {
+            const int row = pass_out_row<R, NS, TPC>(tc, t, r);
+            sm[(SW ? swizzle_row<R0>(row, CT * sizeof(cplx_t<T>)) : row) * CT + cl] = v[t * R + r];
+        }
 }
 
 // The real outputs of one thread of a C2R pass: columns c0 (and c1 when has1)
@@ -274,6 +278,16 @@ __device__ __forceinline__ cplx_t<T> deriv_mul_packed(int order, double w, int k
     return mk(m * Z.x, m * Z.y);
 }
 
+// Whether the exchange after the first pass is swizzled (swizzle_row): FP64 lengths
+// 1024 and 512 y passes 926 -> 890 us (1024 x 1024 x 256), x passes 141 / 135 -> 135 /
+// 128 us (512 x 512 x 128), derivatives FP32 512 x 128 x 65 20.5 -> 18.6 us; not in FP64
+// derivatives of length 512, whose two transforms it makes spill (32.8 -> 34.7 us).
+template <typename T, int L, int MODE>
+constexpr bool fft_swizzled()
+{
+    return !(MODE == FFT_DERIV && L == 512 && sizeof(T) == 8);
+}
+
 // Batch and column within it of column g < total; 64-bit division only where needed.
 __device__ __forceinline__ void split_column(long long g, int ccols, long long total, int& b, int& c)
 {
@@ -302,6 +316,7 @@ __global__ void __launch_bounds__(THREADS, (fft_min_ctas<T, TIO, L, MODE, THREAD
     using C = cplx_t<T>;
     using S = FftShape<T, L, THREADS, SMALL>;
     constexpr int R0 = S::R0, R1 = S::R1, R2 = S::R2, NP = S::NP, TPC = S::TPC, CT = S::CT;
+    constexpr bool SW = fft_swizzled<T, L, MODE>();
     extern __shared__ __align__(16) unsigned char fft_smem[];
     C* sm = reinterpret_cast<C*>(fft_smem);
     const C* tw = static_cast<const C*>(a.tw);
@@ -445,9 +460,9 @@ __global__ void __launch_bounds__(THREADS, (fft_min_ctas<T, TIO, L, MODE, THREAD
     // --------------------------------------------------- later passes --
     if constexpr (NP >= 2) {
         if constexpr (MODE == FFT_C2R || MODE == FFT_C2R_ADJ) __syncthreads();  // pass 0 read shared memory
-        pass_to_smem<T, L, R0, 1, TPC, CT, R0>(sm, tc, cl, v);
+        pass_to_smem<T, L, R0, 1, TPC, CT, R0, SW>(sm, tc, cl, v);
         __syncthreads();
-        pass_from_smem<T, L, R1, R0, DIR, TPC, CT, R0>(sm, tw, tc, cl, v);
+        pass_from_smem<T, L, R1, R0, DIR, TPC, CT, R0, SW>(sm, tw, tc, cl, v);
     }
     if constexpr (NP >= 3) {
         __syncthreads();
@@ -468,7 +483,7 @@ __global__ void __launch_bounds__(THREADS, (fft_min_ctas<T, TIO, L, MODE, THREAD
             for (int r = 0; r < RL; ++r)
                 v[t * RL + r] = deriv_mul_packed<T, L>(a.deriv_order, a.deriv_w, pass_out_row<RL, NSL, TPC>(tc, t, r),
                                                        v[t * RL + r]);
-        fft_inverse_mirror<T, L, TPC, R0, R1, R2, NP>(sm, CT, tw, tc, cl, v);
+        fft_inverse_mirror<T, L, TPC, R0, R1, R2, NP, SW>(sm, CT, tw, tc, cl, v);
         if (valid) {
             TIO* out = static_cast<TIO*>(a.out) + out_base;
 #pragma unroll
@@ -609,6 +624,7 @@ __global__ void __launch_bounds__(THREADS) fft_pipe_kernel(FftArgs a, long long 
     using S = FftShape<T, L, THREADS, SMALL>;
     using PS = PipeShape<T, TIO, L, THREADS, SMALL>;
     constexpr int R0 = S::R0, R1 = S::R1, R2 = S::R2, NP = S::NP, TPC = S::TPC, CT = S::CT;
+    constexpr bool SW = fft_swizzled<T, L, MODE>();
     extern __shared__ __align__(16) unsigned char fft_smem[];
     const C* tw = static_cast<const C*>(a.tw);
     const int tc = threadIdx.x / CT;
@@ -710,9 +726,9 @@ __global__ void __launch_bounds__(THREADS) fft_pipe_kernel(FftArgs a, long long 
 
         // ------------------------------------------------ later passes --
         if constexpr (NP >= 2) {
-            pass_to_smem<T, L, R0, 1, TPC, CT, R0>(sm, tc, cl, v);
+            pass_to_smem<T, L, R0, 1, TPC, CT, R0, SW>(sm, tc, cl, v);
             __syncthreads();
-            pass_from_smem<T, L, R1, R0, DIR, TPC, CT, R0>(sm, tw, tc, cl, v);
+            pass_from_smem<T, L, R1, R0, DIR, TPC, CT, R0, SW>(sm, tw, tc, cl, v);
         }
         if constexpr (NP >= 3) {
             __syncthreads();
@@ -733,7 +749,7 @@ __global__ void __launch_bounds__(THREADS) fft_pipe_kernel(FftArgs a, long long 
                 for (int r = 0; r < RL; ++r)
                     v[t * RL + r] = deriv_mul_packed<T, L>(a.deriv_order, a.deriv_w,
                                                            pass_out_row<RL, NSL, TPC>(tc, t, r), v[t * RL + r]);
-            fft_inverse_mirror<T, L, TPC, R0, R1, R2, NP>(sm, CT, tw, tc, cl, v);
+            fft_inverse_mirror<T, L, TPC, R0, R1, R2, NP, SW>(sm, CT, tw, tc, cl, v);
             if (valid) {
                 TIO* out = static_cast<TIO*>(a.out) + out_base;
 #pragma unroll
