@@ -283,7 +283,7 @@ __device__ __forceinline__ cplx_t<T> deriv_mul_packed(int order, double w, int k
 // 128 us (512 x 512 x 128), derivatives FP32 512 x 128 x 65 20.5 -> 18.6 us; not in FP64
 // derivatives of length 512, whose two transforms it makes spill (32.8 -> 34.7 us).
 template <typename T, int L, int MODE>
-constexpr bool fft_swizzled()
+__host__ __device__ constexpr bool fft_swizzled()
 {
     return !(MODE == FFT_DERIV && L == 512 && sizeof(T) == 8);
 }
