@@ -11,10 +11,11 @@
 // few whole rows, all their elements in shared memory, and runs
 //   1. the interior solves of all its (row, element) vectors side by side:
 //      phi = V diag(1 / (lam - sigma)) V^-1 f as two products on the FP64 tensor
-//      cores (m8n8k4), four complex vectors per warp; the first product's results
-//      are the second one's A operand as they stand, the order of its k index
-//      being put into the B fragments; the second product has two more output
-//      rows, D0 V and DN V, which give the end slopes;
+//      cores (m8n8k4), four complex vectors per warp (elements of up to 34 points;
+//      longer ones: all warps on each vector, multi_solve_wide); the first
+//      product's results are the second one's A operand as they stand, the order
+//      of its k index being put into the B fragments; the second product has two
+//      more output rows, D0 V and DN V, which give the end slopes;
 //   2. the interface sweep, one row per warp, real and imaginary part on a lane
 //      each: the pivots come from the plan, so a step is one multiply-add;
 //   3. the combination and one coalesced store.
@@ -35,8 +36,22 @@ namespace helm {
 namespace {
 
 struct MultiSmem {
-    size_t x, rec, piv, mul, z, sl, total;
+    size_t x, y, rec, piv, mul, z, sl, total;
 };
+
+// Elements of more than this many interior points take multi_solve_wide.
+constexpr int MULTI_WARP_N = 32;
+// Vectors of one round of multi_solve_wide: four m-tiles (four complex vectors
+// each) share every B fragment that a warp loads.
+constexpr int MULTI_WIDE = 16;
+
+// Doubles between the rows of multi_solve_wide's intermediate (8 mod 16: the
+// double2 reads of an A fragment, eight rows by four, touch every bank twice).
+__host__ __device__ inline int multi_wide_stride(int n)
+{
+    const int kp = (n + 7) / 8 * 8;
+    return kp & 8 ? kp : kp + 8;
+}
 
 template <typename TS>
 __host__ __device__ inline MultiSmem multi_smem(int R, int Ns, int P, int n)
@@ -46,6 +61,11 @@ __host__ __device__ inline MultiSmem multi_smem(int R, int Ns, int P, int n)
     const size_t nv = (size_t)R * Ns, kp = (n + 7) / 8 * 8;
     L.x = o;
     o += (nv * P * 2 * sizeof(TS) + 15) / 16 * 16;
+    L.y = o;                                     // first product's results (multi_solve_wide)
+    if (n > MULTI_WARP_N) {
+        const size_t v = nv < MULTI_WIDE ? (nv + 3) / 4 * 4 : MULTI_WIDE;
+        o += v * 2 * multi_wide_stride(n) * sizeof(double);
+    }
     L.rec = o;                                   // 1 / (lam - sigma) of each row
     o += R * kp * sizeof(double);
     L.z = o;                                     // right-hand sides, then interface values
@@ -118,6 +138,91 @@ __device__ __forceinline__ void multi_solve4(const MultiArgs& a, TS* x, const do
         }
 }
 
+// The interior solves of all of a CTA's vectors by all of its warps, for elements of
+// more than MULTI_WARP_N points: a warp takes one n-tile of a product (8 of the n
+// columns) for MULTI_WIDE vectors at a time, so it carries 8 accumulators a lane
+// whatever n is, every B fragment serves four m-tiles, and the few vectors of a short
+// grid still occupy all warps.  The first product's results pass through y, the
+// solutions go over the right-hand sides in x.  With whole-row accumulators
+// (multi_solve4 at 8 and 16 tiles) these sizes spilled 250 bytes to 4.8 KB a thread
+// and one warp walked 40 to 180 KB of fragments by itself: FP64 solves of 256 Fourier
+// points by 2 x 67 took 53.5 us and by 6 x 103 113, walking the elements in turn 29.6
+// and 71.6; with this 20.4 and 28.7.
+template <typename TS, bool SLOPES>
+__device__ __forceinline__ void multi_solve_wide(const MultiArgs& a, TS* x, const double* rec, double* sl, double* y,
+                                                 int nv, int R, int lane, int warp, int nwarp)
+{
+    constexpr int G = MULTI_WIDE / 4;
+    const int g = lane >> 2, q = lane & 3;
+    const int n = a.n, nt = (n + 7) >> 3, kp = nt * 8, ys = multi_wide_stride(n);
+    const int no = SLOPES ? (n + 9) >> 3 : nt;
+    for (int c0 = 0; c0 < nv; c0 += MULTI_WIDE) {
+        const int groups = min(G, (nv - c0 + 3) >> 2);
+        // this lane's vector of each group, real or imaginary part (rows past the end: the first vector's, unused)
+        const TS* row[G];
+        bool live[G];
+#pragma unroll
+        for (int i = 0; i < G; ++i) {
+            const int v = c0 + 4 * i + (g >> 1);
+            live[i] = v < nv;
+            row[i] = x + ((size_t)(live[i] ? v : 0) * a.P + 1) * 2 + (g & 1);
+        }
+        for (int t = warp; t < nt; t += nwarp) {
+            const double* b = a.m1 + (size_t)t * 2 * nt * 32 + lane;
+            double c[G][2];
+#pragma unroll
+            for (int i = 0; i < G; ++i) c[i][0] = c[i][1] = 0.0;
+#pragma unroll 4
+            for (int kk = 0; kk < 2 * nt; ++kk) {
+                const double bv = __ldg(b + kk * 32);
+                const int k = 4 * kk + q;
+#pragma unroll
+                for (int i = 0; i < G; ++i)
+                    if (i < groups) dmma_8x8x4(c[i][0], c[i][1], (live[i] && k < n) ? (double)row[i][2 * k] : 0.0, bv);
+            }
+#pragma unroll
+            for (int i = 0; i < G; ++i)
+                if (i < groups) {
+                    const double* rc = rec + (size_t)(live[i] ? (c0 + 4 * i + (g >> 1)) % R : 0) * kp + 8 * t + 2 * q;
+                    *reinterpret_cast<double2*>(y + (size_t)(8 * i + g) * ys + 8 * t + 2 * q) =
+                        make_double2(c[i][0] * rc[0], c[i][1] * rc[1]);
+                }
+        }
+        __syncthreads();
+        for (int t = warp; t < no; t += nwarp) {
+            const double* b = a.m2 + (size_t)t * 2 * nt * 32 + lane;
+            double o[G][2];
+#pragma unroll
+            for (int i = 0; i < G; ++i) o[i][0] = o[i][1] = 0.0;
+#pragma unroll 2
+            for (int kt = 0; kt < nt; ++kt) {
+                const double b0 = __ldg(b + (size_t)kt * 64), b1 = __ldg(b + (size_t)kt * 64 + 32);
+#pragma unroll
+                for (int i = 0; i < G; ++i)
+                    if (i < groups) {
+                        const double2 av = *reinterpret_cast<const double2*>(y + (size_t)(8 * i + g) * ys + 8 * kt + 2 * q);
+                        dmma_8x8x4(o[i][0], o[i][1], av.x, b0);
+                        dmma_8x8x4(o[i][0], o[i][1], av.y, b1);
+                    }
+            }
+#pragma unroll
+            for (int i = 0; i < G; ++i) {
+                if (!live[i]) continue;
+                const int v = c0 + 4 * i + (g >> 1);
+                TS* out = x + ((size_t)v * a.P + 1) * 2 + (g & 1);
+#pragma unroll
+                for (int s = 0; s < 2; ++s) {
+                    const int j = 8 * t + 2 * q + s;
+                    if (j < n) out[2 * j] = (TS)o[i][s];
+                    else if (SLOPES && j < n + 2) sl[(size_t)v * 4 + 2 * (j - n) + (g & 1)] = o[i][s];
+                }
+            }
+        }
+        __syncthreads();  // y is overwritten by the next round
+    }
+}
+
+// NT: tiles of 8 interior points a warp's accumulators hold (multi_solve4); 0: multi_solve_wide.
 template <typename TS, int NT, bool ADJ>
 __global__ void __launch_bounds__(256) multi_rows_kernel(MultiArgs a)
 {
@@ -126,6 +231,7 @@ __global__ void __launch_bounds__(256) multi_rows_kernel(MultiArgs a)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     const MultiSmem L = multi_smem<TS>(R, Ns, P, n);
     TS* x = reinterpret_cast<TS*>(multi_raw + L.x);  // vector v = element * R + row
+    double* y = reinterpret_cast<double*>(multi_raw + L.y);
     double* rec = reinterpret_cast<double*>(multi_raw + L.rec);
     double* z = reinterpret_cast<double*>(multi_raw + L.z);
     double* sl = reinterpret_cast<double*>(multi_raw + L.sl);
@@ -167,9 +273,18 @@ __global__ void __launch_bounds__(256) multi_rows_kernel(MultiArgs a)
     cp_async_wait_all();
     __syncthreads();
 
+    auto interior_solves = [&]() {
+        if constexpr (NT == 0) {
+            multi_solve_wide<TS, !ADJ>(a, x, rec, sl, y, nv, R, lane, warp, nwarp);
+        } else {
+            for (int v0 = 4 * warp; v0 < nv; v0 += 4 * nwarp)
+                multi_solve4<TS, NT, !ADJ>(a, x, rec, sl, v0, nv, R, lane);
+            __syncthreads();
+        }
+    };
+
     if constexpr (!ADJ) {
-        for (int v0 = 4 * warp; v0 < nv; v0 += 4 * nwarp) multi_solve4<TS, NT, true>(a, x, rec, sl, v0, nv, R, lane);
-        __syncthreads();
+        interior_solves();
         for (int r = warp; r < nr; r += nwarp) {
             const int grp = a.grp_of_row[r0 + r];
             const double d0ur = a.homs[grp * 4 + 1];
@@ -295,8 +410,7 @@ __global__ void __launch_bounds__(256) multi_rows_kernel(MultiArgs a)
             x[2 * (size_t)e + 1] = (TS)((double)x[2 * (size_t)e + 1] + w[1] * c0 + w[3] * cN);
         }
         __syncthreads();
-        for (int v0 = 4 * warp; v0 < nv; v0 += 4 * nwarp) multi_solve4<TS, NT, false>(a, x, rec, sl, v0, nv, R, lane);
-        __syncthreads();
+        interior_solves();
         for (int e = threadIdx.x; e < nv * P; e += blockDim.x) {
             const int j = e / seg, i = e - j * seg;
             if (i >= live) continue;
@@ -324,7 +438,8 @@ int run_multi(MultiArgs a, cudaStream_t s)
     const int most = (a.nrows + 2 * 148 - 1) / (2 * 148);
     if (R > most) R = most;
     if (R < 1) R = 1;
-    while (R > 1 && multi_smem<TS>(R, a.Ns, a.P, a.n).total > 72 * 1024) --R;
+    // three CTAs an SM by shared memory, two where all warps share each vector
+    while (R > 1 && multi_smem<TS>(R, a.Ns, a.P, a.n).total > (NT == 0 ? 110 : 72) * 1024) --R;
     a.rows_per_cta = R;
     const size_t smem = multi_smem<TS>(R, a.Ns, a.P, a.n).total;
     if (smem > kMaxSmemPerBlock) return (int)cudaErrorInvalidValue;
@@ -335,7 +450,7 @@ int run_multi(MultiArgs a, cudaStream_t s)
     // Beyond eight CTAs an SM in all, four warps each: more CTAs side by side hide
     // one another's barriers (4160 of 2 x 30 x 6 points 43 us, eight warps 53; but
     // 528 of 2 x 25 x 10 15.5 and 14.6).
-    const int threads = (tasks >= 5 && ctas <= 8 * 148) ? 256 : tasks >= 3 ? 128 : 64;
+    const int threads = (NT == 0 || (tasks >= 5 && ctas <= 8 * 148)) ? 256 : tasks >= 3 ? 128 : 64;
     return (int)launch_k(k, dim3(ctas), dim3(threads), smem, s, a);
 }
 
@@ -345,9 +460,8 @@ int multi_dispatch(const MultiArgs& a, cudaStream_t s)
     const int nt = (a.n + 7) / 8;
     if (nt <= 1) return run_multi<TS, 1>(a, s);
     if (nt <= 2) return run_multi<TS, 2>(a, s);
-    if (nt <= 4) return run_multi<TS, 4>(a, s);
-    if (nt <= 8) return run_multi<TS, 8>(a, s);
-    return run_multi<TS, 16>(a, s);
+    if (a.n <= MULTI_WARP_N) return run_multi<TS, 4>(a, s);
+    return run_multi<TS, 0>(a, s);
 }
 
 }  // namespace
