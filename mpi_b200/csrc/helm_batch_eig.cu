@@ -34,6 +34,7 @@
 #include "../../include/helm_b200.h"
 #include "helm_batch_eig.cuh"
 #include "helm_device.cuh"
+#include "helm_kernels.cuh"
 #include "helm_plan.hpp"
 #include "helm_setup.hpp"
 
@@ -635,7 +636,8 @@ int batch_eig_create(int nprob, const int* Nx, const int* N, const double* lambd
     int nsm = 0;
     if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device) == cudaSuccess && nsm > 0) be->nsm = nsm;
     cudaGetLastError();
-    if (cudaFuncSetAttribute(batch_eig_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) {
+    // (1 KB for the kernel's static variables)
+    if (allow_smem(batch_eig_kernel, smem, kMaxSmemPerBlock - 1024) != cudaSuccess) {
         cudaGetLastError();
         be->release();
         delete be;

@@ -363,7 +363,7 @@ static int run_gll_deriv_bulk(const GllDerivArgs& a, cudaStream_t s)
     if (stages < 2) return -1;  // not this kernel
     const size_t smem = L.b_bytes + (size_t)stages * (tile_bytes + sizeof(uint64_t));
     auto k = gll_deriv_bulk_kernel<T, NT>;
-    cudaError_t e = allow_smem(k, smem);
+    cudaError_t e = allow_smem(k, smem, kMaxSmemPerBlock);
     if (e != cudaSuccess) return (int)e;
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
@@ -390,7 +390,7 @@ static int run_gll_deriv_mma(const GllDerivArgs& a, cudaStream_t s)
     if (warps < 1) return (int)cudaErrorInvalidValue;
     const size_t smem = L.b_bytes + (size_t)warps * L.warp_bytes;
     auto k = gll_deriv_mma_kernel<T, NT>;
-    cudaError_t e = allow_smem(k, smem);
+    cudaError_t e = allow_smem(k, smem, kMaxSmemPerBlock);
     if (e != cudaSuccess) return (int)e;
     static std::atomic<unsigned long long> memo{0};
     const long long resident = resident_ctas(k, warps * 32, smem, memo);

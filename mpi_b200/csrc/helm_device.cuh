@@ -395,12 +395,15 @@ inline bool pdl_enabled()
 
 // Host side: allow `k` its dynamic shared memory.  The default limit (48 KB with
 // the kernel's static arrays) needs no call, and a call is a third of a launch's
-// host time; launches are what a small solve costs on the host.
+// host time; launches are what a small solve costs on the host.  The limit belongs to
+// the kernel, not to the launch, and every plan and thread shares it: `most` is the
+// largest size the kernel is ever launched with (0: always with smem), so that
+// no launch lowers the limit another one is about to need.
 template <typename K>
-inline cudaError_t allow_smem(K k, size_t smem)
+inline cudaError_t allow_smem(K k, size_t smem, size_t most = 0)
 {
     if (smem <= 40 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(most > smem ? most : smem));
 }
 
 // Host side: CTAs of `k` the current device holds at once, the grid of a

@@ -798,9 +798,9 @@ __global__ void __launch_bounds__(EpShape<L>::THREADS, 1) eig_solve2d_kernel(Eig
 }
 
 template <typename K>
-cudaError_t prep(K k, size_t smem)
+cudaError_t prep(K k, size_t smem, size_t most = 0)
 {
-    return allow_smem(k, smem);
+    return allow_smem(k, smem, most);
 }
 
 template <int L>
@@ -824,14 +824,17 @@ int run_3d(int pass, const EigArgs& a, cudaStream_t s)
         if constexpr (L >= 64) {
             if (a.split) {
                 using SS = SplitShape<L>;
-                const size_t sms = SS::smem(2) + ((a1.tma && a1.sub) ? (size_t)SS::H * EP_PITCH * sizeof(double) : 0);
-                if ((e = prep(eig_fwd_split_kernel<L>, sms)) != cudaSuccess) return (int)e;
+                // (a second plane: the misfit adjoint's TMA path, up to 128 rows)
+                constexpr size_t plane = L <= 128 ? (size_t)SS::H * EP_PITCH * sizeof(double) : 0;
+                const size_t sms = SS::smem(2) + ((a1.tma && a1.sub) ? plane : 0);
+                if ((e = prep(eig_fwd_split_kernel<L>, sms, SS::smem(2) + plane)) != cudaSuccess) return (int)e;
                 return (int)launch_k(eig_fwd_split_kernel<L>, dim3(2 * a.Ny), dim3(SS::THREADS), sms, s, a1, tm);
             }
         }
         // the misfit adjoint's TMA path stages u_obs's plane beside f's
-        const size_t smf = (a1.tma && a1.sub) ? sm1 + (size_t)L * EP_PITCH * sizeof(double) : sm1;
-        if ((e = prep(eig_fwd_kernel<L>, smf)) != cudaSuccess) return (int)e;
+        constexpr size_t plane = L <= 128 ? (size_t)L * EP_PITCH * sizeof(double) : 0;
+        const size_t smf = (a1.tma && a1.sub) ? sm1 + plane : sm1;
+        if ((e = prep(eig_fwd_kernel<L>, smf, sm1 + plane)) != cudaSuccess) return (int)e;
         return (int)launch_k(eig_fwd_kernel<L>, dim3(a.Ny), dim3(S::THREADS), smf, s, a1, tm);
     }
     if (pass == 2) {

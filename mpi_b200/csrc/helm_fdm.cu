@@ -19,6 +19,7 @@
 // time (every matrix load feeds RPW rows).  Lane l owns fold index l + 32 t.
 #include "helm_device.cuh"
 #include "helm_fdm.cuh"
+#include "helm_kernels.cuh"
 
 #include <cooperative_groups.h>
 #include <cstdint>
@@ -1158,7 +1159,7 @@ static int run_slab(const FdmArgs& a, const SlabArgs& sa, int nkx, cudaStream_t 
 {
     auto k = a.adjoint ? slab_kernel<L, true> : slab_kernel<L, false>;
     const size_t smem = slab_smem_bytes(L, sa.HS);
-    cudaError_t e = allow_smem(k, smem);
+    cudaError_t e = allow_smem(k, smem, kMaxSmemPerBlock);
     if (e != cudaSuccess) return (int)e;
     return (int)launch_k(k, dim3(2 * nkx), dim3(SLAB_WARPS * 32), smem, s, a, sa);
 }
@@ -1180,7 +1181,7 @@ bool slab_fits(int Ny, int P, int ld)
 {
     if (ld != SLAB_LD || (Ny != 64 && Ny != 128 && Ny != 256)) return false;
     const int H0 = (P + 1) / 2, HS = H0 | 1;
-    return slab_smem_bytes(Ny, HS) <= 232448;
+    return slab_smem_bytes(Ny, HS) <= kMaxSmemPerBlock;
 }
 
 // ============================== refined solve on the tensor cores ==

@@ -543,7 +543,7 @@ static int run_rows(const RowArgs& a, cudaStream_t s)
 {
     auto k = rows_kernel<TS, TF, NSLOT, METHOD, REFINE, ADJ>;
     const RowSmem L = row_smem_layout<TS, TF, METHOD, REFINE>(a.n, a.ldf);
-    cudaError_t e = allow_smem(k, L.total);
+    cudaError_t e = allow_smem(k, L.total, kMaxSmemPerBlock);
     if (e != cudaSuccess) return (int)e;
     int grid = a.ngroups;
     if (METHOD == 2) {

@@ -443,7 +443,7 @@ int run_multi(MultiArgs a, cudaStream_t s)
     a.rows_per_cta = R;
     const size_t smem = multi_smem<TS>(R, a.Ns, a.P, a.n).total;
     if (smem > kMaxSmemPerBlock) return (int)cudaErrorInvalidValue;
-    cudaError_t e = allow_smem(k, smem);
+    cudaError_t e = allow_smem(k, smem, kMaxSmemPerBlock);
     if (e != cudaSuccess) return (int)e;
     const int tasks = (R * a.Ns + 3) / 4;
     const int ctas = (a.nrows + R - 1) / R;
