@@ -424,6 +424,19 @@ inline long long resident_ctas(K k, int threads, size_t smem, std::atomic<unsign
     return n;
 }
 
+// launch_alone: an ordinary launch.  A kernel that calls no pdl_enter() and is launched
+// so shares the SMs neither with the kernel before it nor with the one after it.
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_alone(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    return cudaLaunchKernelEx(&cfg, k, ((KArgs)args)...);
+}
+
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_k(void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args)
 {

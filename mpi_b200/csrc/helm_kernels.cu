@@ -580,11 +580,14 @@ static int rows_dispatch_prec(int method, int prec, const RowArgs& a, cudaStream
 // thread per row.  The forward sweep writes the modified right-hand side in
 // place and the elimination coefficients to `cprime`; the backward sweep reads
 // both.  Consecutive threads take consecutive rows, so every step's loads fall
-// on lines the previous step brought into L1.
+// on lines the previous step brought into L1.  That takes all of an SM's L1, so the
+// kernel runs alone (launch_alone): with CTAs of the FFT passes before or after it
+// resident, their shared memory is L1 that it lacks, and 32 x 32 x 600 points took
+// 730 us instead of 287 (FP32, pipelined passes of 128 threads), 128 x 128 x 600 2400
+// instead of 354 with the passes that the tuner picks.
 template <typename T>
 __global__ void __launch_bounds__(128) thomas_kernel(ThomasArgs a)
 {
-    pdl_enter();
     using C = cplx_t<T>;
     const long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= a.nrows) return;
@@ -908,7 +911,7 @@ static int thomas_dispatch(const ThomasArgs& a, cudaStream_t s)
     if (a.Nz <= 512) return run_thomas_warp<T, 16>(a, s);
     const long long blocks = (a.nrows + 127) / 128;
     if (blocks <= 0) return 0;
-    return (int)launch_k(thomas_kernel<T>, dim3((unsigned)blocks), dim3(128), 0, s, a);
+    return (int)launch_alone(thomas_kernel<T>, dim3((unsigned)blocks), dim3(128), 0, s, a);
 }
 
 int launch_thomas(int prec, const ThomasArgs& a, cudaStream_t s)

@@ -1,0 +1,34 @@
+"""Finite-difference solves of more than 512 points in z (thomas_kernel): the whole
+solve costs no more than its stages one after another, whatever shape the FFT passes
+around the row solves have."""
+import pytest
+import torch
+
+from mpi_b200 import Helmholtz3DFD
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("variant", [0, 1, 4, 5])
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_row_solves_keep_their_cache(cuda, precision, variant):
+    p = Helmholtz3DFD(32, 32, 600, 0.0, 1.0, 0.0, 1.0, 0.0, 1.0, Lambda=20.0, precision=precision)
+    p.set_launch_variants([variant] * 4, 0)
+    f = torch.randn(32, 32, 600, dtype=torch.float64, device=cuda)
+    out = torch.empty_like(f)
+    whole, stages = [], []
+    for _ in range(10):
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        for _ in range(10):
+            p.SolvePDE(f, out=out)
+        b.record()
+        b.synchronize()
+        whole.append(a.elapsed_time(b) / 10.0)
+    # (an event between the stages keeps each of them to itself)
+    p.enable_stage_timing(True)
+    for _ in range(10):
+        p.SolvePDE(f, out=out)
+        stages.append(sum(p.stage_times().values()))
+    # the fastest of each; rows short of cache took 2.3 times the sum
+    assert min(whole) < 1.4 * min(stages)
