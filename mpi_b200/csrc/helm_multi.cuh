@@ -22,7 +22,7 @@ struct MultiArgs {
     const double* sigma;      // [groups]
     const double* hom;        // [groups][2][P] forward homogeneous solutions ul, ur
     const double* homs;       // [groups][4] their end slopes D0.ul, D0.ur, DN.ul, DN.ur
-    // factors of the interface system (multi_interface): [groups][Ns + 1] reciprocal
+    // factors of the interface system (launch_multi_interface): [groups][Ns + 1] reciprocal
     // pivots; periodic: followed by the correction eta [Ns] and its weight
     const double* itf;
     const double* d0;         // [P] first and last row of D (adjoint)
@@ -42,10 +42,11 @@ inline size_t multi_fragment_doubles(int n, int outs)
 std::vector<double> multi_fragments1(int n, const double* M1);
 std::vector<double> multi_fragments2(int n, int outs, const double* M2);
 
-// Reciprocal pivots of the interface system of one shift (and the periodic
-// correction) from the end slopes s[4]; out: Ns + 1 values, periodic 2 (Ns + 1).
-void multi_interface(int Ns, bool periodic, const double s[4], double al, double bl, double ar, double br,
-                     double* out);
+// Reciprocal pivots of the interface system of every shift (and the periodic
+// correction) from the end slopes homs [groups][4]; out: multi_interface_doubles a shift.
+inline int multi_interface_doubles(int Ns, bool periodic) { return (periodic ? 2 : 1) * (Ns + 1); }
+int launch_multi_interface(int ngroups, int Ns, bool periodic, const double* homs, double al, double bl, double ar,
+                           double br, double* out, cudaStream_t s);
 
 // spec_double: the spectrum holds doubles (else floats); arithmetic is FP64.
 int launch_multi(bool spec_double, MultiArgs a, cudaStream_t s);

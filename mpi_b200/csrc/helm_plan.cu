@@ -244,10 +244,9 @@ static int setup_adjoint(Plan& p, const std::vector<double>& A0, const std::vect
 // and DN V below it) in fragment order, the factors of every shift's interface
 // system, and, for the adjoint of plans not periodic in the GLL direction, V^T
 // and V^-T (the interface system is transposed in the kernel).
-static int setup_multi(Plan& p, const std::vector<double>& V, const std::vector<double>& Vi,
-                       const std::vector<double>& homs)
+static int setup_multi(Plan& p, const std::vector<double>& V, const std::vector<double>& Vi)
 {
-    const int N = p.N, n = p.n, G = p.ngroups, M = p.Ns + 1, itf = p.periodic ? 2 * M : M;
+    const int N = p.N, n = p.n, G = p.ngroups;
     const std::vector<double>& D = p.gll.D;
     std::vector<double> vs((size_t)(n + 2) * n), vt((size_t)n * n), vit((size_t)n * n);
     std::copy(V.begin(), V.end(), vs.begin());
@@ -262,30 +261,35 @@ static int setup_multi(Plan& p, const std::vector<double>& V, const std::vector<
         vs[(size_t)n * n + j] = (double)s0;
         vs[(size_t)(n + 1) * n + j] = (double)sN;
     }
-    std::vector<double> f((size_t)G * itf);
-    for (int g = 0; g < G; ++g)
-        multi_interface(p.Ns, p.periodic, &homs[(size_t)g * 4], p.bc.alphal, p.bc.betal, p.bc.alphar, p.bc.betar,
-                        &f[(size_t)g * itf]);
     std::vector<int> gor((size_t)p.nrows, 0);
     for (int g = 0; g < G; ++g)
         for (int rr = p.grp_start[g]; rr < p.grp_start[g + 1]; ++rr) gor[p.grp_rows[rr]] = g;
-    // one allocation and copy for all of it
-    const std::vector<double> parts[5] = {multi_fragments1(n, Vi.data()), multi_fragments2(n, n + 2, vs.data()), f,
+    // one allocation for all of it and one copy for the transforms; the interface
+    // factors are worked out where they stay
+    const std::vector<double> parts[4] = {multi_fragments1(n, Vi.data()), multi_fragments2(n, n + 2, vs.data()),
                                           p.periodic ? std::vector<double>() : multi_fragments1(n, vt.data()),
                                           p.periodic ? std::vector<double>() : multi_fragments2(n, n, vit.data())};
-    double** const dst[5] = {&p.d_mm1, &p.d_mm2, &p.d_itf, &p.d_mm1_adj, &p.d_mm2_adj};
+    double** const dst[4] = {&p.d_mm1, &p.d_mm2, &p.d_mm1_adj, &p.d_mm2_adj};
     std::vector<double> all;
-    size_t at[5];
-    for (int i = 0; i < 5; ++i) {
+    size_t at[4];
+    for (int i = 0; i < 4; ++i) {
         at[i] = all.size();
         all.insert(all.end(), parts[i].begin(), parts[i].end());
         all.resize((all.size() + 15) / 16 * 16, 0.0);
     }
+    const size_t itf = (size_t)G * multi_interface_doubles(p.Ns, p.periodic);
     double* base = nullptr;
     int st;
-    if ((st = p.upload((void**)&base, all.data(), all.size() * sizeof(double)))) return st;
+    if ((st = p.alloc((void**)&base, (all.size() + itf) * sizeof(double)))) return st;
+    cudaError_t e = cudaMemcpy(base, all.data(), all.size() * sizeof(double), cudaMemcpyHostToDevice);
+    if (e != cudaSuccess) return set_cuda_error(e, "upload");
+    for (int i = 0; i < 4; ++i) *dst[i] = parts[i].empty() ? nullptr : base + at[i];
+    p.d_itf = base + all.size();
+    e = (cudaError_t)launch_multi_interface(G, p.Ns, p.periodic, p.d_homs, p.bc.alphal, p.bc.betal, p.bc.alphar,
+                                            p.bc.betar, p.d_itf, 0);
+    if (e != cudaSuccess) return set_cuda_error(e, "interface factors");
     if ((st = p.upload((void**)&p.d_grp_of_row, gor.data(), gor.size() * sizeof(int)))) return st;
-    for (int i = 0; i < 5; ++i) *dst[i] = parts[i].empty() ? nullptr : base + at[i];
+    if ((e = cudaStreamSynchronize(0)) != cudaSuccess) return set_cuda_error(e, "interface factors");
     if (!p.periodic) p.adj_ready = true;
     p.multi = true;
     return HELM_OK;
@@ -651,11 +655,13 @@ static int setup_plan(Plan& p)
         if ((st = p.upload((void**)&p.d_status, &zero, sizeof(int)))) return st;
     }
     if ((st = p.upload((void**)&p.d_D2full, D2.data(), (size_t)N * N * sizeof(double)))) return st;
-    // refinement: interior D2 column-major with leading dimension ld
-    std::vector<double> d2t((size_t)n * ld, 0.0);
-    for (int k = 0; k < n; ++k)
-        for (int i = 0; i < n; ++i) d2t[(size_t)k * ld + i] = A0[i * n + k];
-    if ((st = p.upload((void**)&p.d_d2t, d2t.data(), d2t.size() * sizeof(double)))) return st;
+    // refinement in rows_kernel: interior D2 column-major with leading dimension ld
+    if (lu || p.Ns == 1) {
+        std::vector<double> d2t((size_t)n * ld, 0.0);
+        for (int k = 0; k < n; ++k)
+            for (int i = 0; i < n; ++i) d2t[(size_t)k * ld + i] = A0[i * n + k];
+        if ((st = p.upload((void**)&p.d_d2t, d2t.data(), d2t.size() * sizeof(double)))) return st;
+    }
     auto up_mat = [&](const std::vector<double>& h, void** d) -> int {
         if (fd) return p.upload(d, h.data(), h.size() * sizeof(double));
         std::vector<float> f(h.begin(), h.end());
@@ -685,7 +691,7 @@ static int setup_plan(Plan& p)
         if (p.packed_elems == 0 && (st = setup_adjoint(p, A0, lam, V, Vi, prec_code, homs))) return st;
         if ((st = setup_fast(p, A0, prec_code))) return st;
     } else if (!lu) {
-        if ((st = setup_multi(p, V, Vi, homs))) return st;
+        if ((st = setup_multi(p, V, Vi))) return st;
     }
     if (!p.fast && rows_smem_bytes(p.method, prec_code, n, p.ld) > kMaxSmemPerBlock) {
         g_last_error = "GLL size too large for the row-solve kernel at this precision";
