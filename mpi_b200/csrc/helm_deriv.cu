@@ -198,10 +198,9 @@ __global__ void gll_deriv_mma_kernel(GllDerivArgs a, GdMmaLayout L)
 // (mbarrier-tracked); each of the GB_WARPS warps multiplies one 8-row m-tile
 // of the current tile on the FP64 tensor cores (the folded products of
 // gll_deriv_mma_kernel), writes its outputs over its own input rows, and the
-// finished tile goes back to global memory as one bulk store.  A tile whose
-// byte count is not a multiple of 16 (odd P and an odd row count at the end)
-// moves its last bytes (at most one FP64 value, three FP32 ones) with plain loads
-// and stores.
+// finished tile goes back to global memory as one bulk store.  Bulk copies move
+// multiples of 16 bytes: the rows are a multiple of four in number (a power of two of
+// Fourier points, at least four), the last tile's as well.
 constexpr int GB_WARPS = 8;
 constexpr int GB_ROWS = 8 * GB_WARPS;
 
@@ -228,10 +227,10 @@ __global__ void __launch_bounds__(GB_WARPS * 32, 1) gll_deriv_bulk_kernel(GllDer
     };
     auto issue = [&](int i) {  // thread 0: tile i of this CTA into stage i % stages
         const long long t = tile_of(i);
-        const uint32_t bulk = bytes_of(t) & ~15u;
+        const uint32_t bytes = bytes_of(t);
         uint64_t* bar = &full[i % stages];
-        mbar_arrive_expect_tx(bar, bulk);
-        bulk_load(stage + (size_t)(i % stages) * tile_elems, in + t * GB_ROWS * P, bulk, bar);
+        mbar_arrive_expect_tx(bar, bytes);
+        bulk_load(stage + (size_t)(i % stages) * tile_elems, in + t * GB_ROWS * P, bytes, bar);
     };
     // the first loads go out before the B fragments are built
     if (threadIdx.x == 0) {
@@ -270,9 +269,6 @@ __global__ void __launch_bounds__(GB_WARPS * 32, 1) gll_deriv_bulk_kernel(GllDer
             failed_at = i;
             break;
         }
-        const int all = nr * P, tail = (int)((bytes & 15u) / sizeof(T));  // values past the bulk copy
-        if ((int)threadIdx.x < tail) cur[all - 1 - threadIdx.x] = in[t * GB_ROWS * P + all - 1 - threadIdx.x];
-        __syncthreads();
         if (8 * warp < nr) {
             double cs[NT][2], ca[NT][2];
 #pragma unroll
@@ -322,9 +318,8 @@ __global__ void __launch_bounds__(GB_WARPS * 32, 1) gll_deriv_bulk_kernel(GllDer
         fence_proxy_async_smem();  // the outputs, written through the generic proxy, go out by bulk store
         __syncthreads();
         if (threadIdx.x == 0) {
-            bulk_store(out + t * GB_ROWS * P, cur, bytes & ~15u);
+            bulk_store(out + t * GB_ROWS * P, cur, bytes);
             tma_store_commit();
-            for (int i1 = 1; i1 <= tail; ++i1) out[t * GB_ROWS * P + all - i1] = cur[all - i1];
             // refill the stage of tile i - 1: its store, issued one iteration
             // ago, has read its shared memory once at most this one is pending
             if (i >= 1 && issued < nmine) {
@@ -374,10 +369,10 @@ static int run_gll_deriv_bulk(const GllDerivArgs& a, cudaStream_t s)
     return (int)launch_k(k, dim3((unsigned)grid), dim3(GB_WARPS * 32), smem, s, a, L, stages);
 }
 
-// The packed layout with 16-byte aligned arrays: the bulk-copy kernel.
+// The packed layout with 16-byte aligned arrays and rows in fours: the bulk-copy kernel.
 static bool gll_deriv_packed(const GllDerivArgs& a)
 {
-    return a.x_stride == (long long)a.rows_per_x * a.P && a.elem_stride == (long long)a.nx * a.x_stride &&
+    return a.nrows % 4 == 0 && a.x_stride == (long long)a.rows_per_x * a.P && a.elem_stride == (long long)a.nx * a.x_stride &&
            (reinterpret_cast<uintptr_t>(a.in) & 15) == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0;
 }
 
