@@ -172,7 +172,8 @@ __global__ void __launch_bounds__(ROW_WARPS * 32) rows_kernel(RowArgs a)
     using CS = cplx_t<TS>;
     using CF = cplx_t<TF>;
     extern __shared__ __align__(16) unsigned char row_smem[];
-    const int n = a.n, P = a.P, ld = a.ldf, Ns = a.Ns;
+    const int n = a.n, P = a.P, ld = a.ldf;
+    const int Ns = METHOD == 2 ? 1 : a.Ns;  // FDM with several elements: multi_rows_kernel
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const RowSmem Lay = row_smem_layout<TS, TF, METHOD, REFINE>(n, ld);
     TF* sMat = reinterpret_cast<TF*>(row_smem + Lay.mat);
@@ -558,8 +559,9 @@ static int run_rows(const RowArgs& a, cudaStream_t s)
 template <int NSLOT>
 static int rows_dispatch_prec(int method, int prec, const RowArgs& a, cudaStream_t s)
 {
-    if (a.adjoint) {  // transposed solve: FDM with one element (several: launch_multi)
-        if (method != 2 || a.Ns > 1) return (int)cudaErrorInvalidValue;
+    if (method == 2 && a.Ns > 1) return (int)cudaErrorInvalidValue;  // launch_multi
+    if (a.adjoint) {  // transposed solve: FDM
+        if (method != 2) return (int)cudaErrorInvalidValue;
         if (prec == 0) return run_rows<double, double, NSLOT, 2, false, true>(a, s);
         if (prec == 1) return run_rows<float, float, NSLOT, 2, false, true>(a, s);
         return run_rows<double, float, NSLOT, 2, true, true>(a, s);

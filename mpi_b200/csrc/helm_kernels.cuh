@@ -56,9 +56,7 @@ struct FftArgs {
     // when set, the pass writes 0 to *zero_out first (the lambda sum of the same
     // solve's last pass starts from it; no separate memset)
     double* zero_out;
-    // C2R only: spectral derivative, the half-spectrum row k is multiplied by
-    // (i deriv_w K)^deriv_order on load, K = k below L/2 and -L/2 at L/2
-    // (0: no derivative)
+    // FFT_DERIV only: order 1 or 2 and the wavenumber of one period
     int deriv_order;
     double deriv_w;
     // R2C only (non-pipelined kernel): when set, the transformed input is

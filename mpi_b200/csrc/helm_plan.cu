@@ -488,7 +488,9 @@ static int setup_plan(Plan& p)
     // shared memory up to 129 points at every precision
     const int fold_ld = 32 * (((n / 2 + n % 2) + 31) / 32);
     const bool fold_fits = p.Ns == 1 && fold_ld <= 64 && fdm_fast_smem_bytes(prec_code, fold_ld) <= kMaxSmemPerBlock;
-    // the unfolded FDM transforms live in shared memory; beyond its capacity use the LU method
+    // the unfolded FDM transforms live in rows_kernel's shared memory; beyond its capacity use
+    // the LU method.  (Several elements run multi_rows_kernel, which would take longer ones; they keep
+    // this limit, and with it their method and their refusals: N up to 103 in FP64 and refined plans)
     if (p.method == HELM_METHOD_FDM && !fold_fits && rows_smem_bytes(2, prec_code, n, p.ld) > kMaxSmemPerBlock)
         p.method = HELM_METHOD_LU;
     if (!(p.method == HELM_METHOD_FDM && fold_fits) && rows_smem_bytes(p.method, prec_code, n, p.ld) > kMaxSmemPerBlock) {
@@ -1290,9 +1292,8 @@ int gll_derivative(Plan& p, int order, const void* u, void* du, cudaStream_t s)
     return HELM_OK;
 }
 
-// Spectral derivative along x (axis 0) or y (axis 1, 3D): a real-to-complex
-// pass along the axis into the spectrum scratch, then the complex-to-real pass
-// back with the multiplier (i 2 pi K / L)^order applied on its load.
+// Spectral derivative along x (axis 0) or y (axis 1, 3D): one pass along the axis
+// (FFT_DERIV), forward transform, multiplier (i 2 pi K / L)^order and inverse.
 int fourier_derivative(Plan& p, int axis, int order, const void* u, void* du, cudaStream_t s)
 {
     if (p.batch > 1) { g_last_error = "derivative of a batched plan"; return HELM_ERR_UNSUPPORTED; }
