@@ -480,15 +480,7 @@ template <typename TS, int NT>
 int run_multi(MultiArgs a, cudaStream_t s)
 {
     auto k = a.adjoint ? multi_rows_kernel<TS, NT, true> : multi_rows_kernel<TS, NT, false>;
-    // Rows per CTA: 64 vectors, two groups of four for each of eight warps, when the
-    // elements are few, while every SM still gets two CTAs.  With 32 vectors a
-    // CTA's fixed costs (plan data, barriers, the sweep) weighed twice as much: 14.6
-    // against 18.6 us (stage, between events) for 1056 rows of 25 x 10 points,
-    // 18.3 against 22.4 for 2112 of 6 x 20; 52 x 10 on 257 rows is the same 14.7.
-    int R = 64 / a.Ns;
-    const int most = (a.nrows + 2 * 148 - 1) / (2 * 148);
-    if (R > most) R = most;
-    if (R < 1) R = 1;
+    int R = multi_rows_per_cta(a.nrows, a.Ns, a.sms);
     // three CTAs an SM by shared memory, two where all warps share each vector
     while (R > 1 && multi_smem<TS>(R, a.Ns, a.P, a.n).total > (NT == 0 ? 110 : 72) * 1024) --R;
     a.rows_per_cta = R;
@@ -501,7 +493,7 @@ int run_multi(MultiArgs a, cudaStream_t s)
     // Beyond eight CTAs an SM in all, four warps each: more CTAs side by side hide
     // one another's barriers (4160 of 2 x 30 x 6 points 43 us, eight warps 53; but
     // 528 of 2 x 25 x 10 15.5 and 14.6).
-    const int threads = (NT == 0 || (tasks >= 5 && ctas <= 8 * 148)) ? 256 : tasks >= 3 ? 128 : 64;
+    const int threads = (NT == 0 || (tasks >= 5 && ctas <= 8 * a.sms)) ? 256 : tasks >= 3 ? 128 : 64;
     return (int)launch_k(k, dim3(ctas), dim3(threads), smem, s, a);
 }
 

@@ -14,6 +14,7 @@ struct MultiArgs {
     void* spec;               // complex [Ns][nrows][P] (elem_stride between elements)
     long long elem_stride;    // complex elements
     int P, n, Ns, nrows;
+    int sms;                  // multiprocessors of the plan's device
     int rows_per_cta;         // set by launch_multi
     const int* grp_of_row;    // shift group of each spectrum row
     const double* m1;         // first transform, fragment order (multi_fragments)
@@ -47,6 +48,17 @@ std::vector<double> multi_fragments2(int n, int outs, const double* M2);
 inline int multi_interface_doubles(int Ns, bool periodic) { return (periodic ? 2 : 1) * (Ns + 1); }
 int launch_multi_interface(int ngroups, int Ns, bool periodic, const double* homs, double al, double bl, double ar,
                            double br, double* out, cudaStream_t s);
+
+// Rows per CTA before the shared memory bounds them: 64 vectors, two groups of four for
+// each of eight warps, when the elements are few, while every SM still gets two CTAs.
+// With 32 vectors a CTA's fixed costs (plan data, barriers, the sweep) weighed twice as
+// much: 14.6 against 18.6 us (stage, between events) for 1056 rows of 25 x 10 points,
+// 18.3 against 22.4 for 2112 of 6 x 20; 52 x 10 on 257 rows is the same 14.7.
+inline int multi_rows_per_cta(int nrows, int Ns, int sms)
+{
+    const int r = 64 / Ns, most = (nrows + 2 * sms - 1) / (2 * sms), rows = r < most ? r : most;
+    return rows < 1 ? 1 : rows;
+}
 
 // spec_double: the spectrum holds doubles (else floats); arithmetic is FP64.
 int launch_multi(bool spec_double, MultiArgs a, cudaStream_t s);

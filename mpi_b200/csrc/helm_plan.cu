@@ -290,6 +290,10 @@ static int setup_multi(Plan& p, const std::vector<double>& V, const std::vector<
     if (e != cudaSuccess) return set_cuda_error(e, "interface factors");
     if ((st = p.upload((void**)&p.d_grp_of_row, gor.data(), gor.size() * sizeof(int)))) return st;
     if ((e = cudaStreamSynchronize(0)) != cudaSuccess) return set_cuda_error(e, "interface factors");
+    if (cudaDeviceGetAttribute(&p.sms, cudaDevAttrMultiProcessorCount, p.device) != cudaSuccess || p.sms < 1) {
+        cudaGetLastError();
+        p.sms = 148;
+    }
     if (!p.periodic) p.adj_ready = true;
     p.multi = true;
     return HELM_OK;
@@ -989,6 +993,7 @@ static int run_pipeline(Plan& p, const void* in, const double* gl, const double*
         ma.n = p.n;
         ma.Ns = p.Ns;
         ma.nrows = (int)p.nrows;
+        ma.sms = p.sms;
         ma.grp_of_row = p.d_grp_of_row;
         ma.m1 = adjoint ? p.d_mm1_adj : p.d_mm1;
         ma.m2 = adjoint ? p.d_mm2_adj : p.d_mm2;

@@ -26,7 +26,7 @@ struct Plan {
     int precision = HELM_FP64, method = HELM_METHOD_AUTO;
     int io_bytes = 8, sweeps = 1;
     long long x_stride = 0, elem_stride = 0, bc_x_stride = 0;
-    int device = 0;
+    int device = 0, sms = 148;   // multiprocessors of the device (launch shapes)
     GllSetup gll;
 
     // rows grouped by shift
