@@ -142,7 +142,10 @@ class _PlanBase:
                                   or not g.is_contiguous()):
                 raise ValueError(f"{nm} must be a contiguous CUDA float64 tensor of shape {bshape}")
         if out is None:
-            out = torch.empty_like(f, memory_format=torch.contiguous_format)
+            # (half the host time of torch.empty; a subclass would make u one as well)
+            plain = type(f) is torch.Tensor or type(f) is torch.nn.Parameter
+            out = torch.empty_like(f, memory_format=torch.contiguous_format) if plain else \
+                torch.empty(f.shape, dtype=self.io_dtype, device=f.device)
         elif tuple(out.shape) != tuple(f.shape) or out.dtype != self.io_dtype or not out.is_contiguous():
             raise ValueError("out does not match f")
         st = self._lib.helm_solve(self._plan, fv.data_ptr(), gl.data_ptr() if gl is not None else None,
