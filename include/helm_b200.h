@@ -307,9 +307,9 @@ int helm_plan_set_launch_variants(helm_plan_t plan, const int* fft4, int rows);
 
 /* Launch variant of the spectral derivative passes (helm_fourier_derivative),
  * with the bits of the FFT variants above (bit 2: the persistent pipelined
- * kernel).  -1, the default, picks by transform length and precision:
- * 512-thread CTAs from length 512; below, the radix-8 schedule, pipelined for
- * FP32 plans.  Pipelined shapes whose tile buffers exceed shared memory are
+ * kernel).  -1, the default, picks by axis, transform length and precision: y
+ * passes the radix-8 schedule (lengths 128 and 256), FP64 x passes up to length 256
+ * 128-thread CTAs, the rest 256-thread CTAs; none pipelined.  Pipelined shapes whose tile buffers exceed shared memory are
  * refused with HELM_ERR_CUDA and launch nothing.  Every
  * variant computes the same derivative up to the last bits.  No counterpart in
  * the reference, which has one code path. */

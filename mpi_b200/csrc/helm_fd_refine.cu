@@ -20,11 +20,12 @@ namespace {
 // scale_r * gr at k = Nz - 1 on the right-hand side.
 //
 // A CTA takes RES_PER * 256 consecutive points of one x plane, RES_PER a thread,
-// and a thread fetches all it reads before it computes.  Bound: the reads of the
-// field and the right-hand side, which L2 holds only in part.  One point after
-// another with 64-bit divisions for (i, j, k) took 34.5 us at 256 x 128 x 100
-// (66 MB), this 29 us; marching along x with the planes in registers (2 or 4 a
-// thread) took 30 and 36 us: the registers cost more warps than the reads saved.
+// and a thread fetches all it reads before it computes.  Bound: instruction issue (77 %
+// of the slots, for eight neighbours' addresses and the FP64 arithmetic a point; the
+// 66 MB of 256 x 128 x 100 alone would take 10 us).  One point after another with 64-bit
+// divisions for (i, j, k) took 34.5 us there, this 29 us; marching along x with the
+// planes in registers (2 or 4 a thread) took 30 and 36 us: the registers cost more
+// warps than the reads saved.
 constexpr int RES_PER = 2;
 
 __global__ void __launch_bounds__(256) fd_residual_kernel(FdResidualArgs a)

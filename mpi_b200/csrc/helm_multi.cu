@@ -24,9 +24,9 @@
 // Bound: latency.  The vectors are short (8 interior points and 52 elements in the
 // stock 2D problem, 4.3 MB in all), so what counts is that no step of one element
 // waits for another element's.  One warp walking the elements of a row in turn
-// (rows_kernel, which the LU method keeps) took 92.7 us for the 257 rows of 52 x 10
-// points and 93.6 us for 1056 rows of 25 x 10 (periodic); this kernel 10.0 and
-// 14.8 us, each with the wait for the pass before it (launched ahead of its end).
+// (rows_kernel, which the LU method keeps) took 84.4 us for the 257 rows of 52 x 10
+// points and 96.3 us for 1056 rows of 25 x 10 (periodic); this kernel 14.8 and
+// 14.5 us (the stage between events, as are the other stage times in these files).
 #include "helm_device.cuh"
 #include "helm_kernels.cuh"
 #include "helm_multi.cuh"

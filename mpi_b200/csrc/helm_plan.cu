@@ -786,6 +786,10 @@ static int fft_pass(Plan& p, int L, int mode, int dir, const void* in, void* out
     // radix 16 36.3); FP64 x passes up to 256 on 128-thread CTAs of radix 16
     // (18.0; 256 threads 20.2, radix 8 22.1); the rest on 256 threads (512 x 128 x
     // 65: x 27.6, 512-thread CTAs 33.2; FP32 256 x 256 x 65: x 13.1, radix 8 14.5).
+    // Lengths 512 and 1024, calls in a row, FP64 / FP32 arrays, 256 threads against 512 and
+    // pipelined: x 512 x 256 x 65 48.2 / 29.7 (59.9 / 34.6, 54.2 / 35.9), x 1024 x 128 x 65
+    // 49.4 / 27.7 (59.3 / 28.8, 68.9 / 40.0), y 256 x 512 x 65 57.2 / 36.6 (70.8 / 41.1, 69.0 /
+    // 46.5), y 128 x 1024 x 65 83.9 / 39.8 (93.1 / 45.2, 86.8 / 50.7).
     const int dvar = p.deriv_var >= 0 ? p.deriv_var : stage == 1 ? 2 : (td && L <= 256) ? 1 : 0;
     const int var = mode == FFT_DERIV ? dvar : sub ? (p.fft_var[stage] & ~4) : p.fft_var[stage];
     int e = launch_fft(L, kmode, dir, td, io, a, ccols * nbatch, s, var);
