@@ -261,14 +261,11 @@ __device__ __forceinline__ cplx_t<T> deriv_mul_packed(int order, double w, int k
 // Whether the exchange after the first pass is swizzled (swizzle_row): FP64 lengths
 // 1024 and 512 y passes 926 -> 890 us (1024 x 1024 x 256), x passes 141 / 135 -> 135 /
 // 128 us (512 x 512 x 128), derivatives FP32 512 x 128 x 65 20.5 -> 18.6 us; not in FP64
-// derivatives of length 512, whose two transforms it makes spill (32.8 -> 34.7 us), nor in
-// FP32 complex passes of length 1024 on 512 threads (fft_kernel's THREADS), whose 64
-// registers it exceeds (1024 x 1024 x 64: 124.9 us, swizzled 135.2; 256 threads 149.5 and 139.3).
-template <typename T, int L, int MODE, int THREADS = 0>
+// derivatives of length 512, whose two transforms it makes spill (32.8 -> 34.7 us).
+template <typename T, int L, int MODE>
 __host__ __device__ constexpr bool fft_swizzled()
 {
-    return !(MODE == FFT_DERIV && L == 512 && sizeof(T) == 8) &&
-           !(MODE == FFT_C2C && L == 1024 && sizeof(T) == 4 && THREADS == 512);
+    return !(MODE == FFT_DERIV && L == 512 && sizeof(T) == 8);
 }
 
 // Batch and column within it of column g < total; 64-bit division only where needed.
@@ -285,16 +282,9 @@ __device__ __forceinline__ void split_column(long long g, int ccols, long long t
 
 // Warps an SM has room for: 24 (at most 85 registers a thread), or 16 where 16
 // points of 8 bytes a thread, or an adjoint pass's operands, would spill at that.
-// Complex passes have no pairs to keep in flight: given those registers FP32 ones, and
-// FP64 ones of eight points a thread, hold fewer warps and gain nothing, so the compiler
-// is left to its own count (0), or held to two CTAs of 512 threads at length 1024.
-// 512-thread CTAs of length 512, 1024 x 512 x 64 FP32: 32 registers 59.4 us, 54 71.7;
-// 256 x 512 x 128 FP64: 56 registers 58 us, 75 86; 256 x 256 x 256 FP32 24.5 and 26.6.
 template <typename T, typename TIO, int L, int MODE, int THREADS, int SMALL>
 constexpr int fft_min_ctas()
 {
-    if (MODE == FFT_C2C && (sizeof(T) == 4 || RadixV<L, SMALL>::r0 <= 8))
-        return sizeof(T) == 4 && L == 1024 && THREADS == 512 ? 2 : 0;
     if (THREADS > 256) return 1;
     const bool many = MODE == FFT_C2R_ADJ || (RadixV<L, SMALL>::r0 > 8 && sizeof(TIO) == 8);
     return (many ? 512 : 768) / THREADS;
@@ -306,7 +296,7 @@ __global__ void __launch_bounds__(THREADS, (fft_min_ctas<T, TIO, L, MODE, THREAD
     using C = cplx_t<T>;
     using S = FftShape<T, L, THREADS, SMALL>;
     constexpr int R0 = S::R0, R1 = S::R1, R2 = S::R2, NP = S::NP, TPC = S::TPC, CT = S::CT;
-    constexpr bool SW = fft_swizzled<T, L, MODE, THREADS>();
+    constexpr bool SW = fft_swizzled<T, L, MODE>();
     extern __shared__ __align__(16) unsigned char fft_smem[];
     C* sm = reinterpret_cast<C*>(fft_smem);
     const C* tw = static_cast<const C*>(a.tw);
