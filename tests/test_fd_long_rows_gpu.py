@@ -17,7 +17,9 @@ def test_row_solves_keep_their_cache(cuda, precision, variant):
     f = torch.randn(32, 32, 600, dtype=torch.float64, device=cuda)
     out = torch.empty_like(f)
     whole, stages = [], []
-    for _ in range(10):
+    # the fastest of each counts (rows short of cache took 2.3 times the sum of the
+    # stages); a busy machine gets more tries
+    for _ in range(40):
         a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         a.record()
         for _ in range(10):
@@ -25,10 +27,11 @@ def test_row_solves_keep_their_cache(cuda, precision, variant):
         b.record()
         b.synchronize()
         whole.append(a.elapsed_time(b) / 10.0)
-    # (an event between the stages keeps each of them to itself)
-    p.enable_stage_timing(True)
-    for _ in range(10):
+        # (an event between the stages keeps each of them to itself)
+        p.enable_stage_timing(True)
         p.SolvePDE(f, out=out)
         stages.append(sum(p.stage_times().values()))
-    # the fastest of each; rows short of cache took 2.3 times the sum
+        p.enable_stage_timing(False)
+        if len(whole) >= 6 and min(whole) < 1.4 * min(stages):
+            break
     assert min(whole) < 1.4 * min(stages)
