@@ -631,9 +631,9 @@ static int setup_plan(Plan& p)
     p.nrows = (long long)nkx * Nyf;
     p.elem_spec = p.nrows * N;
     int st;
-    // the spectrum scratch also holds the half spectra of a derivative along y
-    // (Nx x (Ny/2+1) rows per element), larger than the solve's when Nx > Ny,
-    // and the coefficient spectrum of the eigen-basis pipeline (64 per row)
+    // the spectrum scratch also holds the coefficient spectrum of the eigen-basis
+    // pipeline (64 per row); Nx x (Ny/2+1) rows per element, more than a solve needs when
+    // Nx > Ny, is the size that callers of the workspace query know
     p.eig_cand = p.Ns == 1 && !p.periodic && !p.fd && p.bc.alphal == 0.0 && p.bc.alphar == 0.0 &&
                  p.precision != HELM_FP32 && p.method == HELM_METHOD_FDM && (p.batch == 1 || p.dim == 2) &&
                  eig_shape_ok(p.dim, p.Nx, p.Ny, N);
