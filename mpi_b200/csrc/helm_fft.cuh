@@ -282,10 +282,6 @@ __device__ __forceinline__ void split_column(long long g, int ccols, long long t
 
 // Warps an SM has room for: 24 (at most 85 registers a thread), or 16 where 16
 // points of 8 bytes a thread, or an adjoint pass's operands, would spill at that.
-// Complex passes by themselves are faster without the bound (length 512, 1024 x 512 x 64 FP32:
-// 59.4 us at 32 registers, 71.7 bounded), and so are solves of many tiles (437 us
-// against 460), but solves of few tiles are not: 64 x 512 x 33 FP64 54.9 us against 47.7
-// bounded, finite differences of 64 x 512 x 64 FP32 36.2 against 32.4.
 template <typename T, typename TIO, int L, int MODE, int THREADS, int SMALL>
 constexpr int fft_min_ctas()
 {
@@ -294,13 +290,25 @@ constexpr int fft_min_ctas()
     return (many ? 512 : 768) / THREADS;
 }
 
-template <typename T, typename TIO, int L, int DIR, int MODE, int THREADS, int SMALL>
-__global__ void __launch_bounds__(THREADS, (fft_min_ctas<T, TIO, L, MODE, THREADS, SMALL>())) fft_kernel(FftArgs a, long long total_cols)
+// MANY: complex passes of many tiles on 512 threads (length 512; FP32 1024 as well).  They have
+// no pairs to keep in flight: given the registers of the bound above they hold half the
+// warps, and gain only while the tiles are few.  Left to its own count the compiler
+// takes 32 instead of 54 registers (FP32 length 512: 59.4 us a pass of 1024 x 512 x 64,
+// 71.7 bounded) or 56 instead of 75 (FP64, 256 x 512 x 128: 58 and 86 us); two CTAs of length 1024
+// FP32 need its exchange unswizzled (1024 x 1024 x 64: 125 us, 135 swizzled, 162 in one CTA).
+template <typename T, int L, int MODE, int THREADS>
+constexpr bool fft_has_many()
+{
+    return MODE == FFT_C2C && THREADS == 512 && (L == 512 || (L == 1024 && sizeof(T) == 4));
+}
+
+template <typename T, typename TIO, int L, int DIR, int MODE, int THREADS, int SMALL, bool MANY = false>
+__global__ void __launch_bounds__(THREADS, (MANY ? (L == 512 ? 0 : 2) : fft_min_ctas<T, TIO, L, MODE, THREADS, SMALL>())) fft_kernel(FftArgs a, long long total_cols)
 {
     using C = cplx_t<T>;
     using S = FftShape<T, L, THREADS, SMALL>;
     constexpr int R0 = S::R0, R1 = S::R1, R2 = S::R2, NP = S::NP, TPC = S::TPC, CT = S::CT;
-    constexpr bool SW = fft_swizzled<T, L, MODE>();
+    constexpr bool SW = fft_swizzled<T, L, MODE>() && !(MANY && L == 1024);
     extern __shared__ __align__(16) unsigned char fft_smem[];
     C* sm = reinterpret_cast<C*>(fft_smem);
     const C* tw = static_cast<const C*>(a.tw);
@@ -815,6 +823,17 @@ static int run_fft(const FftArgs& a, long long total_cols, cudaStream_t s)
     if (e != cudaSuccess) return (int)e;
     const long long blocks = (total_cols + S::CT - 1) / S::CT;
     if (blocks <= 0) return 0;
+    if constexpr (fft_has_many<T, L, MODE, THREADS>()) {
+        // Beyond two waves of the bounded kernel: whole solves, bounded and this, 64 x 512 x 150 finite
+        // differences FP32 (618 tiles) 73.4 and 69.6 us, 256 x 512 x 33 FP64 (532) 155.9 and 149.9, 1024 x
+        // 512 x 64 FP32 461.7 and 438.0; below it the bounded one: 64 x 512 x 33 FP64 (136) 47.7 and 54.9,
+        // 64 x 512 x 64 finite differences FP32 (264) 32.4 and 36.2
+        static std::atomic<unsigned long long> memo{0};
+        if (blocks > 2 * resident_ctas(k, THREADS, S::smem, memo)) {
+            k = fft_kernel<T, TIO, L, DIR, MODE, THREADS, SMALL, true>;
+            if ((e = allow_smem(k, S::smem)) != cudaSuccess) return (int)e;
+        }
+    }
     return (int)launch_k(k, dim3((unsigned)blocks), dim3(THREADS), S::smem, s, a, total_cols);
 }
 
